@@ -26,6 +26,7 @@
 #ifndef MC3D_ENGINE_CUH
 #define MC3D_ENGINE_CUH
 
+#include <limits.h>
 #include <stdint.h>
 #include <cuda_runtime.h>
 #include "mc3d_rng.h"
@@ -37,7 +38,11 @@ namespace mc3d {
 /* ---------------------------------------------------------------- math policies
  * A policy fixes the transport arithmetic type (real) and how the elementary
  * operations are evaluated, and reads the per-tissue coefficients of the optical
- * table (three float4 per tissue, see photon_step). */
+ * table (three float4 per tissue, see photon_step).  mul(a, b) is a product rounded
+ * on its own; mad(a, b, c) is a b + c, one rounding with fast math and two with the
+ * others.  The step uses these two wherever a product feeds a sum, so which
+ * products fuse is written down and not the compiler's choice: the tallies do not
+ * change with the code around an expression or with the register budget. */
 
 /* The FP32 policies read every coefficient as the float the reference computes
  * per step, precomputed on the host. */
@@ -52,11 +57,12 @@ struct FloatTable {
     static __device__ __forceinline__ float hg_cos(const float4 *tt, float xi)
     {
         const float4 t2 = tt[2];
-        float c = M::div(t2.x, t2.y + t2.z * xi);
-        return tt[1].w * (t2.w - c * c);
+        const float c = M::div(t2.x, M::mad(t2.z, xi, t2.y));
+        return M::mul(tt[1].w, M::mad(-c, c, t2.w));
     }
     /* thresholds of src/mc3d_types.h:11-18, see the constants below */
     static __device__ __forceinline__ bool w_below_threshold(float w) { return w <= 0x1.a36e2ep-14f; }
+    static __device__ __forceinline__ bool w_above_threshold(float w) { return w > 0x1.a36e2ep-14f; }
     static __device__ __forceinline__ bool uz_within(float u) { return u <= 0x1.fffeb0p-1f; }
     static __device__ __forceinline__ float roulette_survivor(float w)
     {
@@ -69,11 +75,17 @@ struct FloatTable {
 
 struct MathExact : FloatTable {
     static constexpr bool kFast = false;
-    /* a product rounded on its own, never fused into a following add */
-    static __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+    static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+    static __device__ __forceinline__ float mad(float a, float b, float c) { return a * b + c; }
     static __device__ __forceinline__ float div(float a, float b) { return a / b; }
     /* a / b where the caller also holds r = 1/b: the exact policy divides */
     static __device__ __forceinline__ float div_r(float a, float b, float) { return a / b; }
+    /* x + u t for a hit, x + us / mu_t for a scattering; us is u or u s */
+    static __device__ __forceinline__ float advance(float x, float us, bool hit, float t, float mu_t,
+                                                    float)
+    {
+        return x + (hit ? us * t : us / mu_t);
+    }
     static __device__ __forceinline__ float sqrt(float x) { return sqrtf(x); }
     static __device__ __forceinline__ float rsqrt(float x) { return 1.0f / sqrtf(x); }
     static __device__ __forceinline__ float log(float x) { return mc3d_xm_logf(x); }
@@ -93,12 +105,18 @@ struct MathExact : FloatTable {
  * operators and functions below map to the approximate hardware paths. */
 struct MathFast : FloatTable {
     static constexpr bool kFast = true;
-    static __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+    static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+    static __device__ __forceinline__ float mad(float a, float b, float c) { return __fmaf_rn(a, b, c); }
     /* every denominator divided here is a direction cosine, a sum of products of
      * cosines and sines, a refractive-index sum or 1 - g + 2 g xi, all far below the
      * 2^126 where __fdividef stops being defined; x / 0 still gives +-inf or NaN */
     static __device__ __forceinline__ float div(float a, float b) { return __fdividef(a, b); }
-    static __device__ __forceinline__ float div_r(float a, float, float r) { return a * r; }
+    static __device__ __forceinline__ float div_r(float a, float, float r) { return __fmul_rn(a, r); }
+    static __device__ __forceinline__ float advance(float x, float us, bool hit, float t, float,
+                                                    float rmu_t)
+    {
+        return __fmaf_rn(us, hit ? t : rmu_t, x);
+    }
     static __device__ __forceinline__ float sqrt(float x) { return sqrtf(x); }
     static __device__ __forceinline__ float rsqrt(float x) { return rsqrtf(x); }
     static __device__ __forceinline__ float log(float x) { return logf(x); }
@@ -126,9 +144,15 @@ struct MathFast : FloatTable {
 struct MathF64 {
     using real = double;
     static constexpr bool kFast = false;
-    static __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+    static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+    static __device__ __forceinline__ double mad(double a, double b, double c) { return a * b + c; }
     static __device__ __forceinline__ double div(double a, double b) { return a / b; }
     static __device__ __forceinline__ double div_r(double a, double b, double) { return a / b; }
+    static __device__ __forceinline__ double advance(double x, double us, bool hit, double t,
+                                                     double mu_t, double)
+    {
+        return x + (hit ? us * t : us / mu_t);
+    }
     static __device__ __forceinline__ double sqrt(double x) { return ::sqrt(x); }
     static __device__ __forceinline__ double rsqrt(double x) { return 1.0 / ::sqrt(x); }
     static __device__ __forceinline__ double log(double x) { return ::log(x); }
@@ -160,6 +184,7 @@ struct MathF64 {
         return (1 + g * g - c * c) / (2 * g);
     }
     static __device__ __forceinline__ bool w_below_threshold(double w) { return w < 0.0001; }
+    static __device__ __forceinline__ bool w_above_threshold(double w) { return w >= 0.0001; }
     static __device__ __forceinline__ bool uz_within(double u) { return u <= 0.99999; }
     static __device__ __forceinline__ double roulette_survivor(double w) { return w / 0.1; }
     static __device__ __forceinline__ double zero_threshold() { return 1 - 0.99999; }
@@ -190,66 +215,64 @@ struct MathF64 {
 #define MC3D_TAB_STRIDE 3 /* float4 per tissue in the optical table */
 
 
-/* src/mc3d_gpu.cu:53-63 */
+/* Voxel index of x along one axis (src/mc3d_gpu.cu:53-63), as a real: exact below
+ * 2^24, NaN for a NaN position.  `pos` is the direction's sign (u >= 0).  The
+ * reference takes i = floor(x / d), steps up when x lies on the upper face, and
+ * keeps a voxel only when x is above its lower face or on it moving up; the two
+ * cases that leave floor's value are tested here. */
 template <class M, class R = typename M::real>
-static __device__ __forceinline__ int grid_coord(R x, R ux, float d_, float rd_)
+static __device__ __forceinline__ R grid_index(R x, bool pos, float d_, float rd_)
 {
     const R d = d_, rd = rd_;
-    /* the index is carried as a float (exact for |i| < 2^24), which saves the
-     * int <-> float conversions of the two face products */
-    R fi = M::floor(M::div_r(x, d, rd));
+    const R fi = M::floor(M::div_r(x, d, rd));
     const R f1 = fi + (R)1;
-    const R hi = f1 * d;
-    const bool up = (x == hi);
-    fi = up ? f1 : fi;
-    const R bmin = up ? hi : fi * d;
-    const bool stay = (x > bmin) || ((x == bmin) && (ux >= 0));
-    return (int)fi - (stay ? 0 : 1);
+    const R lo = M::mul(fi, d);
+    const bool up = pos && x == M::mul(f1, d);
+    const bool down = !(x >= lo) || (!pos && x == lo);
+    const R f = down ? fi - (R)1 : fi;
+    return up ? f1 : f;
 }
+
+/* A voxel index as an int, before the clamp into the grid.  The conversion's own
+ * result for the NaN position of a photon that the quickfix is about to remove (0
+ * in FP32, below the range in FP64) less the face rule's one picks the first
+ * voxel in FP32 and, by wrapping, the last in FP64. */
+static __device__ __forceinline__ int cell_int(float f) { return (int)f; }
+static __device__ __forceinline__ int cell_int(double f) { return f == f ? (int)f : INT_MAX; }
 
 /* src/mc3d_gpu.cu:24-27 with the clamp addressing of the texture (:416-418).
  * With JUMP the lookup reads the packed map (tissue | box radius << 8, one
  * 16-bit load), so the box radius rides in bits 8-15 of the result (0 above
  * the surface, where the tissue is air). */
 template <bool JUMP = false, class R = float>
-static __device__ __forceinline__ int tissue_at(const GeomDev &g, int i, int j, int k, R z, R uz)
+static __device__ __forceinline__ int tissue_at(const GeomDev &g, R fi, R fj, R fk, R z, R uz)
 {
-    int ci = min(max(i, 0), g.nx - 1);
-    int cj = min(max(j, 0), g.ny - 1);
-    int ck = min(max(k, 0), g.nz - 1);
+    const int ci = min(max(cell_int(fi), 0), g.nx - 1);
+    const int cj = min(max(cell_int(fj), 0), g.ny - 1);
+    const int k = max(cell_int(fk), 0);
     int t;
     if (JUMP) {
-        const int rk = min(max(k, 0), g.nz - 1 + MC3D_SAFE_CAP);
+        const int rk = min(k, g.nz - 1 + MC3D_SAFE_CAP);
         /* 32-bit index: plans take merged steps only for maps below 2^32 cells */
         t = __ldg(g.cells + (((uint32_t)rk * (uint32_t)g.ny + (uint32_t)cj) * (uint32_t)g.nx +
                              (uint32_t)ci));
     } else {
+        const int ck = min(k, g.nz - 1);
         t = __ldg(g.tissue + ((int64_t)ck * g.ny + cj) * g.nx + ci);
     }
     return ((z <= 0) && (uz < 0)) ? MC3D_TISSUE_AIR : t;
 }
 
-/* src/mc3d_gpu.cu:29-49.  With r > 0 the box is the cube of voxels within
- * Chebyshev distance r of (i, j, k) instead of the voxel itself.  Each border is
- * a rounded product, as the reference's separate multiply gives it: fused into
- * the subtraction that follows (which the compiler may do where the snapped
- * positions are unused), a photon lying exactly on a face would see its
- * distance to that face as the product's rounding error instead of 0. */
+/* Distance to one face of the step's box along an axis (src/mc3d_gpu.cu:29-49): the
+ * box reaches r voxels beyond the photon's voxel fi on either side.  The border is
+ * a rounded product, as the reference's separate multiply gives it: fused into the
+ * subtraction that follows, a photon lying exactly on a face would see its distance
+ * to that face as the product's rounding error instead of 0. */
 template <class M, class R = typename M::real>
-static __device__ __forceinline__ R intersection(const GeomDev &g, int i, int j, int k, R *x, R ux,
-                                                 R *y, R uy, R *z, R uz, int r = 0)
+static __device__ __forceinline__ R face_distance(R x, R u, R fi, R r, float d, R *border)
 {
-    R border_x = M::mul_rn((R)((ux >= 0) ? (int)((unsigned)i + 1u + r) : i - r), (R)g.dx);
-    R t_x = M::div(border_x - *x, ux);
-    R border_y = M::mul_rn((R)((uy >= 0) ? (int)((unsigned)j + 1u + r) : j - r), (R)g.dy);
-    R t_y = M::div(border_y - *y, uy);
-    R border_z = M::mul_rn((R)((uz >= 0) ? (int)((unsigned)k + 1u + r) : k - r), (R)g.dz);
-    R t_z = M::div(border_z - *z, uz);
-    R t = M::fmin(t_x, M::fmin(t_y, t_z));
-    *x = (t == t_x) ? border_x : *x + ux * t;
-    *y = (t == t_y) ? border_y : *y + uy * t;
-    *z = (t == t_z) ? border_z : *z + uz * t;
-    return t;
+    *border = M::mul(fi + ((u >= 0) ? r + (R)1 : -r), (R)d);
+    return M::div(*border - x, u);
 }
 
 /* src/mc3d_gpu.cu:113-126 */
@@ -267,7 +290,8 @@ static __device__ __forceinline__ bool mirror(R *x, R *ux, float length_)
 template <class R>
 struct PhotonT {
     R x, y, z, ux, uy, uz, W, s;
-    int i, j, k, tissue;
+    R i, j, k; /* voxel index, as a real: the step's borders need no conversion */
+    int tissue;
 };
 
 /* Per-thread tallies live in shared memory, one column per thread, so that the
@@ -309,188 +333,225 @@ struct Acc {
  * coordinate that was not snapped rounded onto a face; the photon then takes
  * zero-length steps until the quickfix at its chunk's end removes it, which is
  * part of the weight the reference loses. */
-template <class M, bool AMAP, bool JUMP = false, class R = typename M::real>
+template <class M, bool AMAP, bool JUMP = false, bool SPLIT_SIN2 = false,
+          class R = typename M::real>
 static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float4 *tab,
                                                    PhotonT<R> &p, uint64_t &rx, uint32_t ra,
                                                    const Acc &acc, R *db_out,
-                                                   uint32_t *fresnel_count,
                                                    unsigned long long *amap, bool *lat_mirror)
 {
     /* per tissue: (mua, mus, g, n), (mu_t, mua/mu_t, 1/mu_t, 1/(2g)),
      * (1-g^2, 1-g, 2g, 1+g^2) -- each the float the reference computes per step */
-    const int tis = JUMP ? (p.tissue & 0xff) : p.tissue;
-    const float4 *tt = tab + MC3D_TAB_STRIDE * tis;
-    R ni = M::n(tt);
-    R nt = ni;
+    const float4 *tt = tab + MC3D_TAB_STRIDE * (JUMP ? (p.tissue & 0xff) : p.tissue);
     const R mu_t = M::mu_t(tt);
+
+    /* the box's nearest face, src/mc3d_gpu.cu:29-49 */
+    const R r = JUMP ? (R)(p.tissue >> 8) : (R)0;
+    R bx, by, bz;
+    const R t_x = face_distance<M>(p.x, p.ux, p.i, r, g.dx, &bx);
+    const R t_y = face_distance<M>(p.y, p.uy, p.j, r, g.dy, &by);
+    const R t_z = face_distance<M>(p.z, p.uz, p.k, r, g.dz, &bz);
+    const R db = M::fmin(t_x, M::fmin(t_y, t_z));
+    *db_out = db;
+
+    /* move to that face or to the interaction, whichever is nearer: one expression
+     * for both, u 1 db or u s / mu_t from the position, snapped to the face hit */
+    const R ds = M::mul(db, mu_t);
+    const bool hit = ds <= p.s;
+    const R m = hit ? (R)1 : p.s;
     const R rmu_t = M::rmu_t(tt);
+    R newx = M::advance(p.x, M::mul(p.ux, m), hit, db, mu_t, rmu_t);
+    R newy = M::advance(p.y, M::mul(p.uy, m), hit, db, mu_t, rmu_t);
+    R newz = M::advance(p.z, M::mul(p.uz, m), hit, db, mu_t, rmu_t);
+    newx = (hit && db == t_x) ? bx : newx;
+    newy = (hit && db == t_y) ? by : newy;
+    newz = (hit && db == t_z) ? bz : newz;
+    R s = p.s - (hit ? ds : p.s);
 
-    R newx = p.x, newy = p.y, newz = p.z;
-    R db = intersection<M>(g, p.i, p.j, p.k, &newx, p.ux, &newy, p.uy, &newz, p.uz,
-                               JUMP ? (p.tissue >> 8) : 0);
-
-    bool hit = db * mu_t <= p.s;
-    R ds = hit ? db * mu_t : p.s;
-    newx = hit ? newx : p.x + M::div_r(p.ux * ds, mu_t, rmu_t);
-    newy = hit ? newy : p.y + M::div_r(p.uy * ds, mu_t, rmu_t);
-    newz = hit ? newz : p.z + M::div_r(p.uz * ds, mu_t, rmu_t);
-    R s = p.s - ds;
-
-    int nexti = grid_coord<M>(newx, p.ux, g.dx, g.rdx);
-    int nextj = grid_coord<M>(newy, p.uy, g.dy, g.rdy);
-    int nextk = grid_coord<M>(newz, p.uz, g.dz, g.rdz);
+    R nexti = grid_index<M>(newx, p.ux >= 0, g.dx, g.rdx);
+    R nextj = grid_index<M>(newy, p.uy >= 0, g.dy, g.rdy);
+    R nextk = grid_index<M>(newz, p.uz >= 0, g.dz, g.rdz);
     int next_tissue = tissue_at<JUMP>(g, nexti, nextj, nextk, newz, p.uz);
-    nt = M::n(tab + MC3D_TAB_STRIDE * (JUMP ? (next_tissue & 0xff) : next_tissue));
 
-    R tr_ux = p.ux, tr_uy = p.uy, tr_uz = p.uz;
+    /* Fresnel, src/mc3d_gpu.cu:226-257.  The index is looked up only where the
+     * tissue changes.  A photon that goes on from a face (hit) takes the new
+     * direction here; without a hit the direction is the scattered one below, and
+     * a frozen photon keeps its own. */
     bool refl = false;
-    if (ni != nt) { /* src/mc3d_gpu.cu:226-257 */
-        R cos_ai = (p.i != nexti) ? p.ux : ((p.j != nextj) ? p.uy : p.uz);
-        cos_ai = M::fabs(cos_ai);
-        cos_ai = (cos_ai > 1) ? 1 : cos_ai;
-        R ni_nt = M::div(ni, nt);
-        /* sin(acos(c)); fast math evaluates it as sqrt((1 - c)(1 + c)), the same
-         * value without the polynomial of acosf (and more accurate near c = 1) */
-        R sin_ai = M::kFast ? M::sqrt(((R)1 - cos_ai) * ((R)1 + cos_ai))
-                            : M::sin(M::acos(cos_ai));
-        R sin_at = ni_nt * sin_ai;
-        R cos_at = M::sqrt((R)1 - sin_at * sin_at);
-        R R1 = M::div(sin_ai * cos_at - cos_ai * sin_at, sin_ai * cos_at + cos_ai * sin_at);
-        R R2 = M::div(cos_ai * cos_at - sin_ai * sin_at, cos_ai * cos_at + sin_at * sin_at);
-        R Rf = 0.5 * R1 * R1 * ((R)1 + R2 * R2); /* 0.5 is a double literal there too */
-        Rf = (sin_at > 1) ? 1 : Rf;
-        Rf = (ni == nt) ? 0 : Rf;
-        R lat = ni_nt; /* scale of the transmitted lateral cosines */
-        if (M::kFast && M::fabs((R)1 - sin_at * sin_at) < MC3D_NEAR_CRITICAL_F) {
-            /* Near the critical angle 1 - sin_at^2 cancels in float and R is steep:
-             * the same formulas in FP64, sin_ai from cos_ai directly, and the
-             * transmitted direction renormalised in FP64. */
-            const double c = cos_ai;
-            const double rn = (double)ni / (double)nt;
-            const double si = sqrt((1.0 - c) * (1.0 + c));
-            const double st = rn * si;
-            const double ca = sqrt(fmax((1.0 - st) * (1.0 + st), 0.0));
-            const double R1 = (si * ca - c * st) / (si * ca + c * st);
-            const double R2 = (c * ca - si * st) / (c * ca + st * st);
-            Rf = (st >= 1.0) ? (R)1 : (R)(0.5 * R1 * R1 * (1.0 + R2 * R2));
-            const bool xa = p.i != nexti;
-            const bool ya = !xa && p.j != nextj;
-            const bool za = !xa && !ya && p.k != nextk;
-            const double ax = xa ? 0.0 : (double)p.ux;
-            const double ay = ya ? 0.0 : (double)p.uy;
-            const double az = za ? 0.0 : (double)p.uz;
-            const double lat2 = rn * rn * (ax * ax + ay * ay + az * az);
-            const double sc = 1.0 / sqrt(ca * ca + lat2);
-            cos_at = (R)(ca * sc);
-            lat = (R)(rn * sc);
+    if (JUMP ? ((next_tissue ^ p.tissue) & 0xff) != 0 : next_tissue != p.tissue) {
+        const R ni = M::n(tt);
+        const R nt = M::n(tab + MC3D_TAB_STRIDE * (JUMP ? (next_tissue & 0xff) : next_tissue));
+        if (ni != nt) {
+            const bool mx = p.i != nexti, my = p.j != nextj, mz = p.k != nextk;
+            R cos_ai = mx ? p.ux : (my ? p.uy : p.uz);
+            cos_ai = M::fabs(cos_ai);
+            cos_ai = (cos_ai > 1) ? 1 : cos_ai;
+            const R ni_nt = M::div(ni, nt);
+            /* sin(acos(c)); fast math evaluates it as sqrt((1 - c)(1 + c)), the same
+             * value without the polynomial of acosf (and more accurate near c = 1) */
+            const R sin_ai = M::kFast ? M::sqrt(M::mul((R)1 - cos_ai, (R)1 + cos_ai))
+                                      : M::sin(M::acos(cos_ai));
+            const R sin_at = M::mul(ni_nt, sin_ai);
+            R cos_at = M::sqrt(M::mad(-sin_at, sin_at, (R)1));
+            const R sc = M::mul(sin_ai, cos_at), cc = M::mul(cos_ai, cos_at);
+            const R R1 = M::div(M::mad(-cos_ai, sin_at, sc), M::mad(cos_ai, sin_at, sc));
+            const R R2 = M::div(M::mad(-sin_ai, sin_at, cc), M::mad(sin_at, sin_at, cc));
+            /* 0.5 is a double literal there too */
+            R Rf = 0.5 * R1 * R1 * M::mad(R2, R2, (R)1);
+            Rf = (sin_at > 1) ? 1 : Rf;
+            R lat = ni_nt; /* scale of the transmitted lateral cosines */
+            if (M::kFast && M::fabs(M::mad(-sin_at, sin_at, (R)1)) < MC3D_NEAR_CRITICAL_F) {
+                /* Near the critical angle 1 - sin_at^2 cancels in float and R is steep:
+                 * the same formulas in FP64, sin_ai from cos_ai directly, and the
+                 * transmitted direction renormalised in FP64. */
+                const double c = cos_ai;
+                const double rn = (double)ni / (double)nt;
+                const double si = sqrt((1.0 - c) * (1.0 + c));
+                const double st = rn * si;
+                const double ca = sqrt(fmax((1.0 - st) * (1.0 + st), 0.0));
+                const double R1 = (si * ca - c * st) / (si * ca + c * st);
+                const double R2 = (c * ca - si * st) / (c * ca + st * st);
+                Rf = (st >= 1.0) ? (R)1 : (R)(0.5 * R1 * R1 * (1.0 + R2 * R2));
+                const bool xa = mx;
+                const bool ya = !xa && my;
+                const bool za = !xa && !ya && mz;
+                const double ax = xa ? 0.0 : (double)p.ux;
+                const double ay = ya ? 0.0 : (double)p.uy;
+                const double az = za ? 0.0 : (double)p.uz;
+                const double lat2 = rn * rn * (ax * ax + ay * ay + az * az);
+                const double sc = 1.0 / sqrt(ca * ca + lat2);
+                cos_at = (R)(ca * sc);
+                lat = (R)(rn * sc);
+            }
+            const float eps = mc3d_rand_co(&rx, ra);
+            refl = eps < Rf;
+            if (hit && mu_t != 0 && !(p.W <= 0)) {
+                const R tx = mx ? M::copysign(cos_at, M::mul(p.ux, cos_at)) : M::mul(p.ux, lat);
+                const R ty = (my && !mx) ? M::copysign(cos_at, M::mul(p.uy, cos_at))
+                                         : M::mul(p.uy, lat);
+                const R tz = (mz && !my && !mx) ? M::copysign(cos_at, M::mul(p.uz, cos_at))
+                                                : M::mul(p.uz, lat);
+                p.ux = refl ? (mx ? -p.ux : p.ux) : tx;
+                p.uy = refl ? (my ? -p.uy : p.uy) : ty;
+                p.uz = refl ? (mz ? -p.uz : p.uz) : tz;
+            }
+            acc[T_FRESNEL] += 1;
         }
-        float eps = mc3d_rand_co(&rx, ra);
-        refl = eps < Rf;
-        tr_ux = refl ? p.ux * ((p.i == nexti) ? 1 : -1)
-                     : ((p.i != nexti) ? M::copysign(cos_at, p.ux * cos_at) : p.ux * lat);
-        tr_uy = refl ? p.uy * ((p.j == nextj) ? 1 : -1)
-                     : (((p.j != nextj) && (p.i == nexti)) ? M::copysign(cos_at, p.uy * cos_at)
-                                                           : p.uy * lat);
-        tr_uz = refl ? p.uz * ((p.k == nextk) ? 1 : -1)
-                     : (((p.k != nextk) && (p.j == nextj) && (p.i == nexti))
-                            ? M::copysign(cos_at, p.uz * cos_at)
-                            : p.uz * lat);
-        (*fresnel_count)++;
     }
+
+    /* the step's draws: roulette, scattering cosine and azimuth, next free path */
+    rx = mc3d_mwc_next(rx, ra);
+    const uint32_t e_rr = (uint32_t)rx;
+    rx = mc3d_mwc_next(rx, ra);
+    const uint32_t e_hg = (uint32_t)rx;
+    rx = mc3d_mwc_next(rx, ra);
+    const uint32_t e_phi = (uint32_t)rx;
+    rx = mc3d_mwc_next(rx, ra);
+    uint32_t e_s = (uint32_t)rx;
 
     /* absorption, src/mc3d_gpu.cu:262-263 */
     R W = p.W;
-    R dW = (mu_t > 0) ? M::albedo_c(tt) * W : 0;
-    R W_before = W;
-    W = W - dW * (R)(!hit);
+    if (!hit) {
+        const R dW = (mu_t > 0) ? M::mul(M::albedo_c(tt), W) : (R)0;
+        W = W - dW;
+    }
     if (AMAP && !hit && mu_t > 0) {
         /* absorption map, the reference's disabled tally (src/mc3d_gpu.cu:265-272):
          * the current voxel clamped into the grid, fixed-point weight removed.  A
          * merged step can end its flight several voxels from where it started, so
          * there the voxel of the interaction point is used. */
-        int ai = min(max(JUMP ? nexti : p.i, 0), g.nx - 1);
-        int aj = min(max(JUMP ? nextj : p.j, 0), g.ny - 1);
-        int ak = min(max(JUMP ? nextk : p.k, 0), g.nz - 1);
-        uint64_t dq = M::qw(W_before) - M::qw(W);
+        const int ai = min(max((int)(JUMP ? nexti : p.i), 0), g.nx - 1);
+        const int aj = min(max((int)(JUMP ? nextj : p.j), 0), g.ny - 1);
+        const int ak = min(max((int)(JUMP ? nextk : p.k), 0), g.nz - 1);
+        const uint64_t dq = M::qw(p.W) - M::qw(W);
         if (dq) atomicAdd(amap + ((int64_t)ak * g.ny + aj) * g.nx + ai, (unsigned long long)dq);
     }
 
-    /* russian roulette, src/mc3d_gpu.cu:275-277 */
-    float eps = mc3d_rand_co(&rx, ra);
-    bool roulette = M::w_below_threshold(W) && (!hit) && (mu_t != 0);
-    if (roulette) {
-        R newW = (eps < MC3D_SURVIVAL_LT_F) ? M::roulette_survivor(W) : (R)0;
-        /* absorbed weight is booked at the photon's end as Q(W0) - Q(W_end) - lost;
-         * a roulette event moves its share from there to the roulette tallies */
-        if (newW == 0) {
-            uint64_t k = M::qw(W);
-            acc[T_RR_KILLED] += k;
-            acc[T_ABSORBED] -= k;
-        } else {
-            uint64_t c = M::qw(newW) - M::qw(W);
-            acc[T_RR_CREATED] += c;
-            acc[T_ABSORBED] += c;
+    /* Russian roulette (src/mc3d_gpu.cu:275-277) and freezing (:303-311), both
+     * behind the one rare test that either needs */
+    if (!M::w_above_threshold(W) || mu_t == 0) {
+        if (M::w_below_threshold(W) && !hit && mu_t != 0) {
+            const float eps = mc3d_u32_to_float_rz(e_rr) * 0x1p-32f;
+            const R newW = (eps < MC3D_SURVIVAL_LT_F) ? M::roulette_survivor(W) : (R)0;
+            /* absorbed weight is booked at the photon's end as Q(W0) - Q(W_end) - lost;
+             * a roulette event moves its share from there to the roulette tallies */
+            if (newW == 0) {
+                uint64_t k = M::qw(W);
+                acc[T_RR_KILLED] += k;
+                acc[T_ABSORBED] -= k;
+            } else {
+                uint64_t c = M::qw(newW) - M::qw(W);
+                acc[T_RR_CREATED] += c;
+                acc[T_ABSORBED] += c;
+            }
+            W = newW;
         }
-        W = newW;
+        if (W <= 0 || mu_t == 0) { /* freeze: the photon stays where it is */
+            p.W = W;
+            p.s = s;
+            *lat_mirror = false;
+            if (!refl && !(p.x > 0 && p.x < g.Lx && p.y > 0 && p.y < g.Ly))
+                *lat_mirror = mirror<M>(&p.x, &p.ux, g.Lx) || mirror<M>(&p.y, &p.uy, g.Ly);
+            return true;
+        }
+        if (!(W > 0)) e_s = 0; /* NaN weight: no free path, -log(1) */
     }
+    p.W = W;
 
     /* Henyey-Greenstein, src/mc3d_gpu.cu:282-294 */
-    R costheta = M::template hg_cos<M>(tt, (R)mc3d_rand_oc(&rx, ra));
-    R sintheta = M::sqrt(1 - costheta * costheta);
-    R phi_divpi = 2 * (R)mc3d_rand_co(&rx, ra);
+    const R xi = (R)(1.0f - mc3d_u32_to_float_rz(e_hg) * 0x1p-32f);
+    const R costheta = M::template hg_cos<M>(tt, xi);
+    /* 1 - cos^2 with one rounding, but with two in the fast merged-step kernel that maps
+     * one geometry's absorption: that kernel has always rounded the square by itself, and
+     * a seeded run repeats its tallies */
+    const R sintheta = M::sqrt(SPLIT_SIN2 ? (R)1 - M::mul(costheta, costheta)
+                                          : M::mad(-costheta, costheta, (R)1));
     R cosphi, sinphi;
-    M::sincospi(phi_divpi, &sinphi, &cosphi);
-    R invsqrt = M::rsqrt(1 - p.uz * p.uz);
-    bool steep = !M::uz_within(M::fabs(p.uz));
-    R sc_ux = !steep ? sintheta * (p.ux * p.uz * cosphi - p.uy * sinphi) * invsqrt +
-                           p.ux * costheta
-                     : sintheta * cosphi;
-    R sc_uy = !steep ? sintheta * (p.uy * p.uz * cosphi + p.ux * sinphi) * invsqrt +
-                           p.uy * costheta
-                     : sintheta * sinphi;
-    R sc_uz = !steep ? -1 * M::sqrt(1 - p.uz * p.uz) * sintheta * cosphi + p.uz * costheta
-                     : M::copysign(costheta, costheta * p.uz);
+    M::sincospi(2 * (R)(mc3d_u32_to_float_rz(e_phi) * 0x1p-32f), &sinphi, &cosphi);
+    const R sin2 = M::mad(-p.uz, p.uz, (R)1);
+    const R invsqrt = M::rsqrt(sin2);
+    const R Ax = M::mad(-p.uy, sinphi, M::mul(M::mul(p.ux, p.uz), cosphi));
+    const R Ay = M::mad(p.ux, sinphi, M::mul(M::mul(p.uy, p.uz), cosphi));
+    R sc_ux = M::mad(p.ux, costheta, M::mul(M::mul(sintheta, Ax), invsqrt));
+    R sc_uy = M::mad(p.uy, costheta, M::mul(M::mul(sintheta, Ay), invsqrt));
+    R sc_uz = M::mad(p.uz, costheta, M::mul(M::mul(-M::sqrt(sin2), sintheta), cosphi));
+    if (!M::uz_within(M::fabs(p.uz))) {
+        sc_ux = M::mul(sintheta, cosphi);
+        sc_uy = M::mul(sintheta, sinphi);
+        sc_uz = M::copysign(costheta, M::mul(costheta, p.uz));
+    }
 
-    R nux = (!hit) ? sc_ux : tr_ux;
-    R nuy = (!hit) ? sc_uy : tr_uy;
-    R nuz = (!hit) ? sc_uz : tr_uz;
+    R nux = (!hit) ? sc_ux : p.ux;
+    R nuy = (!hit) ? sc_uy : p.uy;
+    R nuz = (!hit) ? sc_uz : p.uz;
     const R zero_thresh = M::zero_threshold();
     nux = (M::fabs(nux) < zero_thresh) ? 0 : nux;
     nuy = (M::fabs(nuy) < zero_thresh) ? 0 : nuy;
     nuz = (M::fabs(nuz) < zero_thresh) ? 0 : nuz;
-    R norm = M::rsqrt(nux * nux + nuy * nuy + nuz * nuz);
-    nux *= norm;
-    nuy *= norm;
-    nuz *= norm;
+    const R norm = M::rsqrt(M::mad(nuz, nuz, M::mad(nuy, nuy, M::mul(nux, nux))));
+    p.ux = M::mul(nux, norm);
+    p.uy = M::mul(nuy, norm);
+    p.uz = M::mul(nuz, norm);
 
-    bool freeze = (W <= 0) || (mu_t == 0);
-    p.ux = !freeze ? nux : p.ux;
-    p.uy = !freeze ? nuy : p.uy;
-    p.uz = !freeze ? nuz : p.uz;
-
-    float e2 = mc3d_rand_oc(&rx, ra);
-    R newS = (W > 0) ? -M::log((R)e2) : 0;
-    p.s = (freeze || hit) ? s : newS;
-    p.W = W;
-
-    p.x = !freeze ? newx : p.x;
-    p.y = !freeze ? newy : p.y;
-    p.z = !freeze ? newz : p.z;
+    const R newS = -M::log((R)(1.0f - mc3d_u32_to_float_rz(e_s) * 0x1p-32f));
+    p.s = hit ? s : newS;
+    p.x = newx;
+    p.y = newy;
+    p.z = newz;
 
     /* mirror boundary conditions, short-circuited as in src/mc3d_gpu.cu:330; off the
      * lateral faces both mirrors are no-ops, which one rarely taken branch tests */
-    bool fres_refl = refl;
-    if (!(p.x > 0 && p.x < g.Lx && p.y > 0 && p.y < g.Ly))
-        refl = refl || mirror<M>(&p.x, &p.ux, g.Lx) || mirror<M>(&p.y, &p.uy, g.Ly);
-    *lat_mirror = refl && !fres_refl;
+    if (!refl && !(p.x > 0 && p.x < g.Lx && p.y > 0 && p.y < g.Ly))
+        refl = mirror<M>(&p.x, &p.ux, g.Lx) || mirror<M>(&p.y, &p.uy, g.Ly);
 
-    bool keep = (hit && refl) || freeze;
-    p.i = keep ? p.i : nexti;
-    p.j = keep ? p.j : nextj;
-    p.k = keep ? p.k : nextk;
-    p.tissue = keep ? p.tissue : next_tissue;
-    *db_out = db;
-    return freeze;
+    /* a reflected photon keeps its voxel (src/mc3d_gpu.cu:334-339) */
+    if (!(hit && refl)) {
+        p.i = nexti;
+        p.j = nextj;
+        p.k = nextk;
+        p.tissue = next_tissue;
+    }
+    return false;
 }
 
 /* i, j, k and tissue from the position, as at the start of every launch of
@@ -498,9 +559,9 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
 template <class M, bool JUMP = false, class R = typename M::real>
 static __device__ __forceinline__ void derive_cell(const GeomDev &g, PhotonT<R> &p)
 {
-    p.i = grid_coord<M>(p.x, p.ux, g.dx, g.rdx);
-    p.j = grid_coord<M>(p.y, p.uy, g.dy, g.rdy);
-    p.k = grid_coord<M>(p.z, p.uz, g.dz, g.rdz);
+    p.i = grid_index<M>(p.x, p.ux >= 0, g.dx, g.rdx);
+    p.j = grid_index<M>(p.y, p.uy >= 0, g.dy, g.rdy);
+    p.k = grid_index<M>(p.z, p.uz >= 0, g.dz, g.rdz);
     p.tissue = tissue_at<JUMP>(g, p.i, p.j, p.k, p.z, p.uz);
 }
 
@@ -511,9 +572,9 @@ static __device__ __forceinline__ void derive_cell(const GeomDev &g, PhotonT<R> 
 template <class R>
 static __device__ __forceinline__ bool cell_consistent(const GeomDev &g, const PhotonT<R> &p)
 {
-    const R xl = (R)p.i * (R)g.dx, xh = (R)(p.i + 1) * (R)g.dx;
-    const R yl = (R)p.j * (R)g.dy, yh = (R)(p.j + 1) * (R)g.dy;
-    const R zl = (R)p.k * (R)g.dz, zh = (R)(p.k + 1) * (R)g.dz;
+    const R xl = p.i * (R)g.dx, xh = (p.i + (R)1) * (R)g.dx;
+    const R yl = p.j * (R)g.dy, yh = (p.j + (R)1) * (R)g.dy;
+    const R zl = p.k * (R)g.dz, zh = (p.k + (R)1) * (R)g.dz;
     const bool ox = (p.x > xl && p.x < xh) || (p.x == xl && p.ux >= 0) || (p.x == xh && p.ux < 0);
     const bool oy = (p.y > yl && p.y < yh) || (p.y == yl && p.uy >= 0) || (p.y == yh && p.uy < 0);
     const bool oz = (p.z > zl && p.z < zh) || (p.z == zl && p.uz >= 0) || (p.z == zh && p.uz < 0);
@@ -534,8 +595,11 @@ static __device__ __forceinline__ bool finite_state(const PhotonT<R> &p)
 template <class M, class R = typename M::real>
 static __device__ __forceinline__ R voxel_db(const GeomDev &g, const PhotonT<R> &p)
 {
-    R x = p.x, y = p.y, z = p.z;
-    return intersection<M>(g, p.i, p.j, p.k, &x, p.ux, &y, p.uy, &z, p.uz);
+    R b;
+    const R t_x = face_distance<M>(p.x, p.ux, p.i, (R)0, g.dx, &b);
+    const R t_y = face_distance<M>(p.y, p.uy, p.j, (R)0, g.dy, &b);
+    const R t_z = face_distance<M>(p.z, p.uz, p.k, (R)0, g.dz, &b);
+    return M::fmin(t_x, M::fmin(t_y, t_z));
 }
 
 /* The NaN/Inf/db==0 quickfix run after each 45-step launch (src/mc3d_gpu.cu:343-353);
@@ -560,8 +624,7 @@ template <class M, class R = typename M::real>
 static __device__ __forceinline__ R masked_steps(const GeomDev &g, PhotonT<R> &p, int masked, R db)
 {
     for (int t = 0; t < masked; t++) {
-        R nx_ = p.x, ny_ = p.y, nz_ = p.z;
-        db = intersection<M>(g, p.i, p.j, p.k, &nx_, p.ux, &ny_, p.uy, &nz_, p.uz);
+        db = voxel_db<M>(g, p);
         if (!mirror<M>(&p.x, &p.ux, g.Lx)) mirror<M>(&p.y, &p.uy, g.Ly);
     }
     return db;
@@ -655,23 +718,17 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
     uint32_t ra = 1;
     PhotonT<R> p;
     bool alive = false;
-    int chunk = 0;
-    /* Loop iterations modulo the 45-step chunk.  A photon starts only at tick 0,
-     * as a reference slot starts only at a launch boundary: a lane whose photon
-     * ended waits out the rest of the chunk (the reference's masked steps), so
-     * the lanes of a warp reach their chunk ends on the same iteration. */
-    int tick = 0;
-    uint32_t psteps = 0;
-    uint32_t fresnel = 0;
+    int psteps = 0; /* steps of the photon before its present chunk */
     unsigned long long *amap = nullptr;
 
+    /* One iteration is one 45-step chunk, the reference's launch.  A photon starts
+     * only at a chunk's start, as a reference slot starts only at a launch boundary:
+     * a lane whose photon ended waits out the rest of the chunk (the reference's
+     * masked steps), so the lanes of a warp start, end and refill photons together
+     * and the step loop itself holds nothing but steps. */
     for (;;) {
         if (!alive) {
-            if (tick != 0) {
-                tick = (tick == MC3D_NUM_PHOTON_STEPS - 1) ? 0 : tick + 1;
-                continue;
-            }
-            if (left == 0) {
+            while (left == 0) {
                 if (P.cancel && *((volatile const int *)P.cancel)) break;
                 int64_t gs = (int64_t)atomicAdd((unsigned long long *)P.work_counter, 1ull);
                 if (gs >= P.total_streams) break;
@@ -688,8 +745,8 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
                 left = jb.per_stream + (local < jb.remainder ? 1 : 0);
                 ra = stream_multiplier(P, local);
                 rx = stream_seed(P, jb, local, ra);
-                if (left == 0) continue;
             }
+            if (left == 0) break;
             const GeomDev &g = ONE_GEOM ? P.geom0 : *gp;
             /* photontrack_reinitialize, src/mc3d_gpu.cu:74-111 */
             if (P.jobs[job].beam == 0) {
@@ -704,33 +761,40 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
             /* specular reflection from air into tissue type 1 (src/mc3d_gpu.cu:67-70, 500) */
             const R n0 = M::n(tab + MC3D_TAB_STRIDE * MC3D_TISSUE_AIR), n1 = M::n(tab + MC3D_TAB_STRIDE);
             R rsp = M::div(n0 - n1, n0 + n1);
-            rsp = rsp * rsp;
+            rsp = M::mul(rsp, rsp);
             p.W = (R)1 - rsp;
             p.s = -M::log((R)mc3d_rand_oc(&rx, ra));
             derive_cell<M, JUMP>(g, p);
-            chunk = 0;
             psteps = 0;
-            fresnel = 0;
             alive = true;
             left--;
         }
 
         const GeomDev &g = ONE_GEOM ? P.geom0 : *gp;
+        /* The chunk's steps, fewer where the step cap comes first.  Merged steps: the
+         * quickfix must see the boundary distance of the reference's one-voxel DDA
+         * for the chunk's last step, not the merged box's (which is never 0 inside a
+         * uniform cube), or merged steps would lose less weight to it than the
+         * reference does.  It is taken from that step's start state, so the loop
+         * stops before that step and goes round once more for it. */
+        const int cap = min(MC3D_NUM_PHOTON_STEPS, (int)P.max_steps - psteps);
+        int stop = JUMP ? min(cap, MC3D_NUM_PHOTON_STEPS - 1) : cap;
+        int chunk = 0;
         R db;
         bool lat_mirror;
         bool froze;
-        /* Merged steps: the quickfix must see the boundary distance of the
-         * reference's one-voxel DDA for the chunk's last step, not the merged
-         * box's (which is never 0 inside a uniform cube), or merged steps would
-         * lose less weight to it than the reference does.  Taken from that
-         * step's start state. */
         bool vzero = false;
-        if (JUMP && chunk == MC3D_NUM_PHOTON_STEPS - 1) vzero = voxel_db<M>(g, p) == 0;
-        froze = photon_step<M, AMAP, JUMP>(g, tab, p, rx, ra, acc, &db, &fresnel, amap,
-                                           &lat_mirror);
-        chunk++;
-        psteps++;
-        tick = (tick == MC3D_NUM_PHOTON_STEPS - 1) ? 0 : tick + 1;
+        for (;;) {
+            do {
+                froze = photon_step<M, AMAP, JUMP, M::kFast && AMAP && JUMP && ONE_GEOM>(
+                    g, tab, p, rx, ra, acc, &db, amap, &lat_mirror);
+                chunk++;
+            } while (!froze && chunk < stop);
+            if (!JUMP || froze || stop == cap) break;
+            vzero = voxel_db<M>(g, p) == 0;
+            stop = cap;
+        }
+        psteps += chunk;
 
         bool done = false;
         uint64_t lost = 0;
@@ -763,10 +827,9 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
                 /* fast math: re-derive only where the stored cell breaks the face rule
                  * (exact math always re-derives, as the reference's relaunch does) */
                 if (!M::kFast || !cell_consistent(g, p)) derive_cell<M, JUMP>(g, p);
-                chunk = 0;
             }
         }
-        if (!done && (int64_t)psteps >= P.max_steps) {
+        if (!done && psteps >= P.max_steps) {
             lost = M::qw(p.W);
             p.W = 0;
             acc[T_CAPPED]++;
@@ -775,8 +838,8 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
         if (done) {
             /* photon_detector, src/mc3d_photons.cu:151-171 */
             const JobDev &jb = P.jobs[job];
-            int ix = grid_coord<M>(p.x, p.ux, g.dx, g.rdx);
-            int iy = grid_coord<M>(p.y, p.uy, g.dy, g.rdy);
+            const int ix = (int)grid_index<M>(p.x, p.ux >= 0, g.dx, g.rdx);
+            const int iy = (int)grid_index<M>(p.y, p.uy >= 0, g.dy, g.rdy);
             bool inside = (ix >= 0) && (iy >= 0) && (ix < g.nx) && (iy < g.ny);
             uint64_t q = M::qw(p.W);
             int64_t bin = jb.bin_offset + (int64_t)iy * g.nx + ix;
@@ -785,7 +848,7 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
                 slot = inside ? T_R_IN : T_R_OUT;
                 if (inside && q) {
                     atomicAdd(P.drs + bin, (unsigned long long)q);
-                    atomicAdd(P.drs_sq + bin, (unsigned long long)M::qw(p.W * p.W));
+                    atomicAdd(P.drs_sq + bin, (unsigned long long)M::qw(M::mul(p.W, p.W)));
                 }
             } else {
                 slot = inside ? T_T_IN : T_T_OUT;
@@ -795,14 +858,13 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
             /* the launch weight 1 - Rsp again, as at the photon's start */
             const R n0 = M::n(tab + MC3D_TAB_STRIDE * MC3D_TISSUE_AIR), n1 = M::n(tab + MC3D_TAB_STRIDE);
             R rsp = M::div(n0 - n1, n0 + n1);
-            rsp = rsp * rsp;
+            rsp = M::mul(rsp, rsp);
             const uint64_t qw0 = M::qw((R)1 - rsp);
             acc[T_W_LAUNCHED] += qw0;
             acc[T_ABSORBED] += qw0 - q - lost;
             acc[T_LOST] += lost;
             acc[T_PHOTONS] += 1;
             acc[T_STEPS] += psteps;
-            acc[T_FRESNEL] += fresnel;
             if (P.photon_log) {
                 int64_t nstream = jb.per_stream + (local < jb.remainder ? 1 : 0);
                 int64_t kphot = nstream - left - 1;
@@ -811,7 +873,7 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
                 r.x = (float)p.x; r.y = (float)p.y; r.z = (float)p.z;
                 r.ux = (float)p.ux; r.uy = (float)p.uy; r.uz = (float)p.uz;
                 r.W = (float)p.W; r.s = (float)p.s;
-                r.steps = psteps;
+                r.steps = (uint32_t)psteps;
                 r.tissue = (uint32_t)(p.tissue & 0xff);
                 r.rng = rx;
                 P.photon_log[pid] = r;
