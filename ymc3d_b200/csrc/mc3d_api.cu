@@ -470,7 +470,9 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
         d.nx = g.nx; d.ny = g.ny; d.nz = g.nz;
         d.dx = (float)g.dx; d.dy = (float)g.dy; d.dz = (float)g.dz;
         /* geometry->length_x = sample_dx*num_x in float (src/mc3d_io.cu:143-145) */
-        d.Lx = d.dx * g.nx; d.Ly = d.dy * g.ny; d.Lz = d.dz * g.nz;
+        d.Lx = d.dx * g.nx; d.Ly = d.dy * g.ny;
+        d.last_x = g.nx - 1; d.last_y = g.ny - 1;
+        d.last_z = g.nz - 1 + (p->jump ? MC3D_SAFE_CAP : 0);
         d.rdx = 1.0f / d.dx; d.rdy = 1.0f / d.dy; d.rdz = 1.0f / d.dz;
         d.tissue = p->d_grids[i];
     }
@@ -523,7 +525,7 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
         for (int t = 0; t < props[i].num_tissue_types; t++) {
             float mua = props[i].mua[t], mus = props[i].mus[t], g = props[i].g[t];
             volatile float mut = mua + mus;
-            volatile float frac = mua / mut, rmut = 1.0f / mut, g2 = g * g, twog = 2 * g;
+            volatile float frac = mut > 0 ? mua / mut : 0.0f, rmut = 1.0f / mut, g2 = g * g, twog = 2 * g;
             volatile float inv2g = 1.0f / twog;
             float4 *e = &tab[props_offset[i] + 3 * t];
             e[0] = make_float4(mua, mus, g, props[i].n[t]);

@@ -50,6 +50,7 @@ struct FloatTable {
     using real = float;
     static __device__ __forceinline__ float n(const float4 *tt) { return tt[0].w; }
     static __device__ __forceinline__ float mu_t(const float4 *tt) { return tt[1].x; }
+    /* mua / mu_t, 0 where mu_t is not positive */
     static __device__ __forceinline__ float albedo_c(const float4 *tt) { return tt[1].y; }
     static __device__ __forceinline__ float rmu_t(const float4 *tt) { return tt[1].z; }
     /* Henyey-Greenstein cos(theta) for the draw xi in (0, 1] (src/mc3d_gpu.cu:282-286) */
@@ -91,9 +92,10 @@ struct MathExact : FloatTable {
     static __device__ __forceinline__ float log(float x) { return mc3d_xm_logf(x); }
     static __device__ __forceinline__ float acos(float x) { return mc3d_xm_acosf(x); }
     static __device__ __forceinline__ float sin(float x) { return mc3d_xm_sinf(x); }
-    static __device__ __forceinline__ void sincospi(float x, float *s, float *c)
+    /* sin and cos of the azimuth 2 pi e 2^-32 */
+    static __device__ __forceinline__ void sincos_draw(uint32_t e, float *s, float *c)
     {
-        mc3d_xm_sincospif(x, s, c);
+        mc3d_xm_sincospif(2 * (mc3d_u32_to_float_rz(e) * 0x1p-32f), s, c);
     }
     static __device__ __forceinline__ float floor(float x) { return floorf(x); }
     static __device__ __forceinline__ float fmin(float a, float b) { return fminf(a, b); }
@@ -122,11 +124,12 @@ struct MathFast : FloatTable {
     static __device__ __forceinline__ float log(float x) { return logf(x); }
     static __device__ __forceinline__ float acos(float x) { return acosf(x); }
     static __device__ __forceinline__ float sin(float x) { return sinf(x); }
-    /* sin/cos(pi x) for x in [0, 2): the SFU's sin/cos on pi (x - 1) in [-pi, pi) */
-    static __device__ __forceinline__ void sincospi(float x, float *s, float *c)
+    /* the SFU's sin/cos on the azimuth less pi, in [-pi, pi) */
+    static __device__ __forceinline__ void sincos_draw(uint32_t e, float *s, float *c)
     {
         float sn, cs;
-        __sincosf(3.14159265358979f * (x - 1.0f), &sn, &cs);
+        const float x = __fmaf_rn(mc3d_u32_to_float_rz(e), 0x1p-31f, -1.0f);
+        __sincosf(__fmul_rn(3.14159265358979f, x), &sn, &cs);
         *s = -sn;
         *c = -cs;
     }
@@ -158,9 +161,9 @@ struct MathF64 {
     static __device__ __forceinline__ double log(double x) { return ::log(x); }
     static __device__ __forceinline__ double acos(double x) { return ::acos(x); }
     static __device__ __forceinline__ double sin(double x) { return ::sin(x); }
-    static __device__ __forceinline__ void sincospi(double x, double *s, double *c)
+    static __device__ __forceinline__ void sincos_draw(uint32_t e, double *s, double *c)
     {
-        ::sincospi(x, s, c);
+        ::sincospi(2 * (double)(mc3d_u32_to_float_rz(e) * 0x1p-32f), s, c);
     }
     static __device__ __forceinline__ double floor(double x) { return ::floor(x); }
     static __device__ __forceinline__ double fmin(double a, double b) { return ::fmin(a, b); }
@@ -173,7 +176,7 @@ struct MathF64 {
     }
     static __device__ __forceinline__ double albedo_c(const float4 *tt)
     {
-        return (double)tt[0].x / mu_t(tt);
+        return mu_t(tt) > 0 ? (double)tt[0].x / mu_t(tt) : 0;
     }
     static __device__ __forceinline__ double rmu_t(const float4 *tt) { return 1.0 / mu_t(tt); }
     template <class M>
@@ -215,22 +218,28 @@ struct MathF64 {
 #define MC3D_TAB_STRIDE 3 /* float4 per tissue in the optical table */
 
 
+/* 1 for a direction that moves up the axis (u >= 0), 0 for one that moves down */
+template <class R>
+static __device__ __forceinline__ R upward(R u)
+{
+    return u >= 0 ? (R)1 : (R)0;
+}
+
 /* Voxel index of x along one axis (src/mc3d_gpu.cu:53-63), as a real: exact below
- * 2^24, NaN for a NaN position.  `pos` is the direction's sign (u >= 0).  The
- * reference takes i = floor(x / d), steps up when x lies on the upper face, and
- * keeps a voxel only when x is above its lower face or on it moving up; the two
- * cases that leave floor's value are tested here. */
+ * 2^24, NaN for a NaN position; up = upward(u).  The reference takes i = floor(x / d),
+ * steps up when x lies on the upper face, and keeps a voxel only when x is above its
+ * lower face or on it moving up.  So floor's value stands unless x lies on the face
+ * that the photon moves through (one voxel on) or, floor's argument having been
+ * rounded up, below the lower face (one voxel back).  Written as arithmetic on 0 and
+ * 1: as predicates the three axes need more of them than a thread has. */
 template <class M, class R = typename M::real>
-static __device__ __forceinline__ R grid_index(R x, bool pos, float d_, float rd_)
+static __device__ __forceinline__ R grid_index(R x, R up, float d_, float rd_)
 {
     const R d = d_, rd = rd_;
     const R fi = M::floor(M::div_r(x, d, rd));
-    const R f1 = fi + (R)1;
-    const R lo = M::mul(fi, d);
-    const bool up = pos && x == M::mul(f1, d);
-    const bool down = !(x >= lo) || (!pos && x == lo);
-    const R f = down ? fi - (R)1 : fi;
-    return up ? f1 : f;
+    const R on_face = x == M::mul(fi + up, d) ? (R)1 : (R)0;
+    const R below = x >= M::mul(fi, d) ? (R)0 : (R)1;
+    return M::mad(on_face, M::mad((R)2, up, (R)-1), fi) - below;
 }
 
 /* A voxel index as an int, before the clamp into the grid.  The conversion's own
@@ -247,17 +256,15 @@ static __device__ __forceinline__ int cell_int(double f) { return f == f ? (int)
 template <bool JUMP = false, class R = float>
 static __device__ __forceinline__ int tissue_at(const GeomDev &g, R fi, R fj, R fk, R z, R uz)
 {
-    const int ci = min(max(cell_int(fi), 0), g.nx - 1);
-    const int cj = min(max(cell_int(fj), 0), g.ny - 1);
-    const int k = max(cell_int(fk), 0);
+    const int ci = min(max(cell_int(fi), 0), g.last_x);
+    const int cj = min(max(cell_int(fj), 0), g.last_y);
+    const int ck = min(max(cell_int(fk), 0), g.last_z);
     int t;
     if (JUMP) {
-        const int rk = min(k, g.nz - 1 + MC3D_SAFE_CAP);
         /* 32-bit index: plans take merged steps only for maps below 2^32 cells */
-        t = __ldg(g.cells + (((uint32_t)rk * (uint32_t)g.ny + (uint32_t)cj) * (uint32_t)g.nx +
+        t = __ldg(g.cells + (((uint32_t)ck * (uint32_t)g.ny + (uint32_t)cj) * (uint32_t)g.nx +
                              (uint32_t)ci));
     } else {
-        const int ck = min(k, g.nz - 1);
         t = __ldg(g.tissue + ((int64_t)ck * g.ny + cj) * g.nx + ci);
     }
     return ((z <= 0) && (uz < 0)) ? MC3D_TISSUE_AIR : t;
@@ -269,9 +276,10 @@ static __device__ __forceinline__ int tissue_at(const GeomDev &g, R fi, R fj, R 
  * subtraction that follows, a photon lying exactly on a face would see its distance
  * to that face as the product's rounding error instead of 0. */
 template <class M, class R = typename M::real>
-static __device__ __forceinline__ R face_distance(R x, R u, R fi, R r, float d, R *border)
+static __device__ __forceinline__ R face_distance(R x, R u, R up, R fi, R r, float d, R *border)
 {
-    *border = M::mul(fi + ((u >= 0) ? r + (R)1 : -r), (R)d);
+    /* fi + r + 1 upward, fi - r downward (whole numbers: exact) */
+    *border = M::mul(fi + M::mad(up, M::mad((R)2, r, (R)1), -r), (R)d);
     return M::div(*border - x, u);
 }
 
@@ -348,9 +356,10 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
     /* the box's nearest face, src/mc3d_gpu.cu:29-49 */
     const R r = JUMP ? (R)(p.tissue >> 8) : (R)0;
     R bx, by, bz;
-    const R t_x = face_distance<M>(p.x, p.ux, p.i, r, g.dx, &bx);
-    const R t_y = face_distance<M>(p.y, p.uy, p.j, r, g.dy, &by);
-    const R t_z = face_distance<M>(p.z, p.uz, p.k, r, g.dz, &bz);
+    const R up_x = upward(p.ux), up_y = upward(p.uy), up_z = upward(p.uz);
+    const R t_x = face_distance<M>(p.x, p.ux, up_x, p.i, r, g.dx, &bx);
+    const R t_y = face_distance<M>(p.y, p.uy, up_y, p.j, r, g.dy, &by);
+    const R t_z = face_distance<M>(p.z, p.uz, up_z, p.k, r, g.dz, &bz);
     const R db = M::fmin(t_x, M::fmin(t_y, t_z));
     *db_out = db;
 
@@ -366,11 +375,11 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
     newx = (hit && db == t_x) ? bx : newx;
     newy = (hit && db == t_y) ? by : newy;
     newz = (hit && db == t_z) ? bz : newz;
-    R s = p.s - (hit ? ds : p.s);
+    const R s = p.s - ds; /* what a hit leaves of the free path */
 
-    R nexti = grid_index<M>(newx, p.ux >= 0, g.dx, g.rdx);
-    R nextj = grid_index<M>(newy, p.uy >= 0, g.dy, g.rdy);
-    R nextk = grid_index<M>(newz, p.uz >= 0, g.dz, g.rdz);
+    R nexti = grid_index<M>(newx, up_x, g.dx, g.rdx);
+    R nextj = grid_index<M>(newy, up_y, g.dy, g.rdy);
+    R nextk = grid_index<M>(newz, up_z, g.dz, g.rdz);
     int next_tissue = tissue_at<JUMP>(g, nexti, nextj, nextk, newz, p.uz);
 
     /* Fresnel, src/mc3d_gpu.cu:226-257.  The index is looked up only where the
@@ -435,6 +444,12 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
                 p.uy = refl ? (my ? -p.uy : p.uy) : ty;
                 p.uz = refl ? (mz ? -p.uz : p.uz) : tz;
             }
+            if (hit && refl) { /* a reflected photon keeps its voxel (:334-339) */
+                nexti = p.i;
+                nextj = p.j;
+                nextk = p.k;
+                next_tissue = p.tissue;
+            }
             acc[T_FRESNEL] += 1;
         }
     }
@@ -451,10 +466,7 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
 
     /* absorption, src/mc3d_gpu.cu:262-263 */
     R W = p.W;
-    if (!hit) {
-        const R dW = (mu_t > 0) ? M::mul(M::albedo_c(tt), W) : (R)0;
-        W = W - dW;
-    }
+    W = W - (hit ? (R)0 : M::mul(M::albedo_c(tt), W));
     if (AMAP && !hit && mu_t > 0) {
         /* absorption map, the reference's disabled tally (src/mc3d_gpu.cu:265-272):
          * the current voxel clamped into the grid, fixed-point weight removed.  A
@@ -488,7 +500,7 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
         }
         if (W <= 0 || mu_t == 0) { /* freeze: the photon stays where it is */
             p.W = W;
-            p.s = s;
+            p.s = hit ? s : p.s - p.s;
             *lat_mirror = false;
             if (!refl && !(p.x > 0 && p.x < g.Lx && p.y > 0 && p.y < g.Ly))
                 *lat_mirror = mirror<M>(&p.x, &p.ux, g.Lx) || mirror<M>(&p.y, &p.uy, g.Ly);
@@ -507,27 +519,41 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
     const R sintheta = M::sqrt(SPLIT_SIN2 ? (R)1 - M::mul(costheta, costheta)
                                           : M::mad(-costheta, costheta, (R)1));
     R cosphi, sinphi;
-    M::sincospi(2 * (R)(mc3d_u32_to_float_rz(e_phi) * 0x1p-32f), &sinphi, &cosphi);
+    M::sincos_draw(e_phi, &sinphi, &cosphi);
     const R sin2 = M::mad(-p.uz, p.uz, (R)1);
     const R invsqrt = M::rsqrt(sin2);
     const R Ax = M::mad(-p.uy, sinphi, M::mul(M::mul(p.ux, p.uz), cosphi));
     const R Ay = M::mad(p.ux, sinphi, M::mul(M::mul(p.uy, p.uz), cosphi));
-    R sc_ux = M::mad(p.ux, costheta, M::mul(M::mul(sintheta, Ax), invsqrt));
-    R sc_uy = M::mad(p.uy, costheta, M::mul(M::mul(sintheta, Ay), invsqrt));
-    R sc_uz = M::mad(p.uz, costheta, M::mul(M::mul(-M::sqrt(sin2), sintheta), cosphi));
-    if (!M::uz_within(M::fabs(p.uz))) {
-        sc_ux = M::mul(sintheta, cosphi);
-        sc_uy = M::mul(sintheta, sinphi);
-        sc_uz = M::copysign(costheta, M::mul(costheta, p.uz));
-    }
-
+    const R sc_ux = M::mad(p.ux, costheta, M::mul(M::mul(sintheta, Ax), invsqrt));
+    const R sc_uy = M::mad(p.uy, costheta, M::mul(M::mul(sintheta, Ay), invsqrt));
+    const R sc_uz = M::mad(p.uz, costheta, M::mul(M::mul(-M::sqrt(sin2), sintheta), cosphi));
     R nux = (!hit) ? sc_ux : p.ux;
     R nuy = (!hit) ? sc_uy : p.uy;
     R nuz = (!hit) ? sc_uz : p.uz;
+
+    /* What few steps need, behind one test: the scattering of a photon along the z
+     * axis, components snapped to zero, and the mirrors at the lateral faces
+     * (short-circuited as in src/mc3d_gpu.cu:330), which are no-ops off them.  A
+     * mirror turns its component before the normalisation, which keeps the sign. */
     const R zero_thresh = M::zero_threshold();
-    nux = (M::fabs(nux) < zero_thresh) ? 0 : nux;
-    nuy = (M::fabs(nuy) < zero_thresh) ? 0 : nuy;
-    nuz = (M::fabs(nuz) < zero_thresh) ? 0 : nuz;
+    const bool steep = !M::uz_within(M::fabs(p.uz));
+    if (steep || M::fabs(nux) < zero_thresh || M::fabs(nuy) < zero_thresh ||
+        M::fabs(nuz) < zero_thresh || !(newx > 0 && newx < g.Lx && newy > 0 && newy < g.Ly)) {
+        if (steep && !hit) {
+            nux = M::mul(sintheta, cosphi);
+            nuy = M::mul(sintheta, sinphi);
+            nuz = M::copysign(costheta, M::mul(costheta, p.uz));
+        }
+        nux = (M::fabs(nux) < zero_thresh) ? 0 : nux;
+        nuy = (M::fabs(nuy) < zero_thresh) ? 0 : nuy;
+        nuz = (M::fabs(nuz) < zero_thresh) ? 0 : nuz;
+        if (!refl && (mirror<M>(&newx, &nux, g.Lx) || mirror<M>(&newy, &nuy, g.Ly)) && hit) {
+            nexti = p.i; /* as after a Fresnel reflection */
+            nextj = p.j;
+            nextk = p.k;
+            next_tissue = p.tissue;
+        }
+    }
     const R norm = M::rsqrt(M::mad(nuz, nuz, M::mad(nuy, nuy, M::mul(nux, nux))));
     p.ux = M::mul(nux, norm);
     p.uy = M::mul(nuy, norm);
@@ -538,19 +564,10 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
     p.x = newx;
     p.y = newy;
     p.z = newz;
-
-    /* mirror boundary conditions, short-circuited as in src/mc3d_gpu.cu:330; off the
-     * lateral faces both mirrors are no-ops, which one rarely taken branch tests */
-    if (!refl && !(p.x > 0 && p.x < g.Lx && p.y > 0 && p.y < g.Ly))
-        refl = mirror<M>(&p.x, &p.ux, g.Lx) || mirror<M>(&p.y, &p.uy, g.Ly);
-
-    /* a reflected photon keeps its voxel (src/mc3d_gpu.cu:334-339) */
-    if (!(hit && refl)) {
-        p.i = nexti;
-        p.j = nextj;
-        p.k = nextk;
-        p.tissue = next_tissue;
-    }
+    p.i = nexti;
+    p.j = nextj;
+    p.k = nextk;
+    p.tissue = next_tissue;
     return false;
 }
 
@@ -559,9 +576,9 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
 template <class M, bool JUMP = false, class R = typename M::real>
 static __device__ __forceinline__ void derive_cell(const GeomDev &g, PhotonT<R> &p)
 {
-    p.i = grid_index<M>(p.x, p.ux >= 0, g.dx, g.rdx);
-    p.j = grid_index<M>(p.y, p.uy >= 0, g.dy, g.rdy);
-    p.k = grid_index<M>(p.z, p.uz >= 0, g.dz, g.rdz);
+    p.i = grid_index<M>(p.x, upward(p.ux), g.dx, g.rdx);
+    p.j = grid_index<M>(p.y, upward(p.uy), g.dy, g.rdy);
+    p.k = grid_index<M>(p.z, upward(p.uz), g.dz, g.rdz);
     p.tissue = tissue_at<JUMP>(g, p.i, p.j, p.k, p.z, p.uz);
 }
 
@@ -596,9 +613,9 @@ template <class M, class R = typename M::real>
 static __device__ __forceinline__ R voxel_db(const GeomDev &g, const PhotonT<R> &p)
 {
     R b;
-    const R t_x = face_distance<M>(p.x, p.ux, p.i, (R)0, g.dx, &b);
-    const R t_y = face_distance<M>(p.y, p.uy, p.j, (R)0, g.dy, &b);
-    const R t_z = face_distance<M>(p.z, p.uz, p.k, (R)0, g.dz, &b);
+    const R t_x = face_distance<M>(p.x, p.ux, upward(p.ux), p.i, (R)0, g.dx, &b);
+    const R t_y = face_distance<M>(p.y, p.uy, upward(p.uy), p.j, (R)0, g.dy, &b);
+    const R t_z = face_distance<M>(p.z, p.uz, upward(p.uz), p.k, (R)0, g.dz, &b);
     return M::fmin(t_x, M::fmin(t_y, t_z));
 }
 
@@ -838,8 +855,8 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
         if (done) {
             /* photon_detector, src/mc3d_photons.cu:151-171 */
             const JobDev &jb = P.jobs[job];
-            const int ix = (int)grid_index<M>(p.x, p.ux >= 0, g.dx, g.rdx);
-            const int iy = (int)grid_index<M>(p.y, p.uy >= 0, g.dy, g.rdy);
+            const int ix = (int)grid_index<M>(p.x, upward(p.ux), g.dx, g.rdx);
+            const int iy = (int)grid_index<M>(p.y, upward(p.uy), g.dy, g.rdy);
             bool inside = (ix >= 0) && (iy >= 0) && (ix < g.nx) && (iy < g.ny);
             uint64_t q = M::qw(p.W);
             int64_t bin = jb.bin_offset + (int64_t)iy * g.nx + ix;

@@ -178,7 +178,7 @@ extern "C" int mc3d_run_noalloc(const mc3d_geom *geom, const mc3d_props *props,
     for (int t = 0; t < nt; t++) {
         float mua = props->mua[t], mus = props->mus[t], g = props->g[t];
         volatile float mut = mua + mus;
-        volatile float frac = mua / mut, rmut = 1.0f / mut, g2 = g * g, twog = 2 * g;
+        volatile float frac = mut > 0 ? mua / mut : 0.0f, rmut = 1.0f / mut, g2 = g * g, twog = 2 * g;
         volatile float inv2g = 1.0f / twog;
         tab[3 * t + 0] = make_float4(mua, mus, g, props->n[t]);
         tab[3 * t + 1] = make_float4(mut, frac, rmut, inv2g);
@@ -188,7 +188,8 @@ extern "C" int mc3d_run_noalloc(const mc3d_geom *geom, const mc3d_props *props,
     memset(&gd, 0, sizeof gd);
     gd.nx = geom->nx; gd.ny = geom->ny; gd.nz = geom->nz;
     gd.dx = (float)geom->dx; gd.dy = (float)geom->dy; gd.dz = (float)geom->dz;
-    gd.Lx = gd.dx * gd.nx; gd.Ly = gd.dy * gd.ny; gd.Lz = gd.dz * gd.nz;
+    gd.Lx = gd.dx * gd.nx; gd.Ly = gd.dy * gd.ny;
+    gd.last_x = gd.nx - 1; gd.last_y = gd.ny - 1; gd.last_z = gd.nz - 1;
     gd.rdx = 1.0f / gd.dx; gd.rdy = 1.0f / gd.dy; gd.rdz = 1.0f / gd.dz;
     gd.tissue = geom->tissue;
     JobDev jd;
