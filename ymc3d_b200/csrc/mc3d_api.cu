@@ -102,7 +102,7 @@ cudaError_t pool_alloc(T **ptr, size_t bytes, int device, cudaStream_t s)
 }
 
 /* bytes of optical tables and geometry descriptors per launch (shared memory:
- * 227 KB per block, less 28 KB of tally columns) */
+ * 227 KB per block, less 34 KB of rows for 256 threads) */
 const int kMaxSharedTable = 192 * 1024;
 const int64_t kMaxAttempts = 4096;       /* seeding attempts per stream before giving up */
 
@@ -221,7 +221,7 @@ struct mc3d_plan {
     int device = 0;
     int math = MC3D_MATH_FAST;
     int variant = 0; /* fast kernel variant bits (MC3D_VARIANT_*) */
-    int block = 256;
+    int block = 0;
     int grid = 0;
     size_t smem = 0;
     cudaStream_t stream = nullptr;
@@ -529,7 +529,7 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
             volatile float inv2g = 1.0f / twog;
             float4 *e = &tab[props_offset[i] + 3 * t];
             e[0] = make_float4(mua, mus, g, props[i].n[t]);
-            e[1] = make_float4(mut, frac, rmut, inv2g);
+            e[1] = make_float4(mut, rmut, frac, inv2g);
             e[2] = make_float4(1 - g2, 1 - g, twog, 1 + g2);
         }
     PLAN_TRY(pool_alloc(&p->d_props, sizeof(float4) * entries, p->device, p->stream));
@@ -598,18 +598,16 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
     PLAN_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, p->device));
     PLAN_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
                                     p->device));
-    p->block = opt.block ? opt.block : 256;
-    p->smem = sizeof(float4) * entries + sizeof(GeomDev) * ngeoms;
-    /* The kernels' static shared memory (28 KB of per-thread tallies) counts
-     * against the 48 KB a block gets without opting in, so the kernels always opt
-     * in, to the device's whole per-block limit: the attribute is per function,
-     * and a lower value would break a live plan that needs more. */
+    /* The kernels always opt in to the device's whole per-block limit of shared
+     * memory: the attribute is per function, and a lower value would break a live
+     * plan that needs more. */
     {
         cudaFuncAttributes fa;
         PLAN_TRY(p->math == MC3D_MATH_FAST    ? attributes_photon_fast(&fa)
                  : p->math == MC3D_MATH_EXACT ? attributes_photon_exact(&fa)
                                               : attributes_photon_f64(&fa));
         const size_t max_dyn = (size_t)smem_optin - fa.sharedSizeBytes;
+        p->smem = photon_smem(entries, ngeoms, opt.block ? opt.block : 128);
         if (p->smem > max_dyn) {
             plan_free(p);
             return fail(MC3D_ERR_CAPACITY, "optical tables and geometry descriptors need %zu B "
@@ -620,10 +618,23 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
                                               : smem_limit_photon_f64(max_dyn));
     }
     p->variant = (p->jump ? 0 : MC3D_VARIANT_VOXEL_STEPS) | (ngeoms == 1 ? MC3D_VARIANT_ONE_GEOM : 0);
+    /* 128 threads, of whose registers an SM holds 20 warps of the fast kernel (16 in
+     * blocks of 256), unless the optical tables, of which each block has a copy, leave
+     * room for more threads in larger blocks */
     int bps = 0;
-    PLAN_TRY(p->math == MC3D_MATH_FAST ? occupancy_photon_fast(p->block, p->smem, &bps, p->variant)
-             : p->math == MC3D_MATH_EXACT ? occupancy_photon_exact(p->block, p->smem, &bps)
-                                          : occupancy_photon_f64(p->block, p->smem, &bps, p->variant));
+    for (int block : {opt.block ? (int)opt.block : 128, opt.block ? 0 : 256}) {
+        if (block == 0) continue;
+        int n = 0;
+        const size_t smem = photon_smem(entries, ngeoms, block);
+        PLAN_TRY(p->math == MC3D_MATH_FAST ? occupancy_photon_fast(block, smem, &n, p->variant)
+                 : p->math == MC3D_MATH_EXACT ? occupancy_photon_exact(block, smem, &n)
+                                              : occupancy_photon_f64(block, smem, &n, p->variant));
+        if (n * block > bps * p->block || p->block == 0) {
+            p->block = block;
+            p->smem = smem;
+            bps = n;
+        }
+    }
     if (bps <= 0) {
         plan_free(p);
         return fail(MC3D_ERR_CAPACITY, "kernel does not fit an SM with block %d", opt.block);

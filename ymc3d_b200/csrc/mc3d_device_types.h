@@ -14,6 +14,10 @@
 /* order of the per-job totals (matches mc3d_totals in include/mc3d.h) */
 #define MC3D_NUM_TOTALS 14
 
+/* words of shared memory per thread of a photon kernel: its tallies, two words of its
+ * stream, and one unused so that the threads of a warp start in different banks */
+#define MC3D_THREAD_WORDS (MC3D_NUM_TOTALS + 3)
+
 /* largest safe distance of the merged-step map, and the number of slices the
  * map adds below the grid (the clamped continuation of the medium) */
 #define MC3D_SAFE_CAP 63

@@ -44,6 +44,82 @@ namespace mc3d {
  * products fuse is written down and not the compiler's choice: the tallies do not
  * change with the code around an expression or with the register budget. */
 
+/* Two values of one step side by side (its x and y axes): the fast policy computes on
+ * both with one instruction, the others one after the other. */
+template <class R>
+struct Pair {
+    R a, b;
+};
+
+template <class M, class R>
+struct PairwiseOps {
+    using P2 = Pair<R>;
+    static __device__ __forceinline__ P2 mul(P2 x, P2 y) { return {M::mul(x.a, y.a), M::mul(x.b, y.b)}; }
+    static __device__ __forceinline__ P2 add(P2 x, P2 y) { return {x.a + y.a, x.b + y.b}; }
+    static __device__ __forceinline__ P2 sub(P2 x, P2 y) { return {x.a - y.a, x.b - y.b}; }
+    static __device__ __forceinline__ P2 mad(P2 x, P2 y, P2 z)
+    {
+        return {M::mad(x.a, y.a, z.a), M::mad(x.b, y.b, z.b)};
+    }
+    static __device__ __forceinline__ P2 div(P2 x, P2 y) { return {M::div(x.a, y.a), M::div(x.b, y.b)}; }
+    static __device__ __forceinline__ P2 div_r(P2 x, P2 y, P2 r)
+    {
+        return {M::div_r(x.a, y.a, r.a), M::div_r(x.b, y.b, r.b)};
+    }
+};
+
+/* FP32 pairs in the packed instructions of sm_100, each rounding as its scalar form */
+struct PackedOps {
+    using P2 = Pair<float>;
+    static __device__ __forceinline__ uint64_t pack(P2 x)
+    {
+        uint64_t r;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x.a), "f"(x.b));
+        return r;
+    }
+    static __device__ __forceinline__ P2 unpack(uint64_t v)
+    {
+        P2 r;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(r.a), "=f"(r.b) : "l"(v));
+        return r;
+    }
+    static __device__ __forceinline__ P2 mul(P2 x, P2 y)
+    {
+        uint64_t r;
+        asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack(x)), "l"(pack(y)));
+        return unpack(r);
+    }
+    static __device__ __forceinline__ P2 add(P2 x, P2 y)
+    {
+        uint64_t r;
+        asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack(x)), "l"(pack(y)));
+        return unpack(r);
+    }
+    static __device__ __forceinline__ P2 sub(P2 x, P2 y)
+    {
+        uint64_t r;
+        asm("sub.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack(x)), "l"(pack(y)));
+        return unpack(r);
+    }
+    static __device__ __forceinline__ P2 mad(P2 x, P2 y, P2 z)
+    {
+        uint64_t r;
+        asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;"
+            : "=l"(r)
+            : "l"(pack(x)), "l"(pack(y)), "l"(pack(z)));
+        return unpack(r);
+    }
+    static __device__ __forceinline__ float rcp(float x)
+    {
+        float r;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+        return r;
+    }
+    /* as __fdividef: the product with the approximate reciprocal */
+    static __device__ __forceinline__ P2 div(P2 x, P2 y) { return mul(x, P2{rcp(y.a), rcp(y.b)}); }
+    static __device__ __forceinline__ P2 div_r(P2 x, P2, P2 r) { return mul(x, r); }
+};
+
 /* The FP32 policies read every coefficient as the float the reference computes
  * per step, precomputed on the host. */
 struct FloatTable {
@@ -51,8 +127,8 @@ struct FloatTable {
     static __device__ __forceinline__ float n(const float4 *tt) { return tt[0].w; }
     static __device__ __forceinline__ float mu_t(const float4 *tt) { return tt[1].x; }
     /* mua / mu_t, 0 where mu_t is not positive */
-    static __device__ __forceinline__ float albedo_c(const float4 *tt) { return tt[1].y; }
-    static __device__ __forceinline__ float rmu_t(const float4 *tt) { return tt[1].z; }
+    static __device__ __forceinline__ float albedo_c(const float4 *tt) { return tt[1].z; }
+    static __device__ __forceinline__ float rmu_t(const float4 *tt) { return tt[1].y; }
     /* Henyey-Greenstein cos(theta) for the draw xi in (0, 1] (src/mc3d_gpu.cu:282-286) */
     template <class M>
     static __device__ __forceinline__ float hg_cos(const float4 *tt, float xi)
@@ -63,19 +139,43 @@ struct FloatTable {
     }
     /* thresholds of src/mc3d_types.h:11-18, see the constants below */
     static __device__ __forceinline__ bool w_below_threshold(float w) { return w <= 0x1.a36e2ep-14f; }
-    static __device__ __forceinline__ bool w_above_threshold(float w) { return w > 0x1.a36e2ep-14f; }
     static __device__ __forceinline__ bool uz_within(float u) { return u <= 0x1.fffeb0p-1f; }
     static __device__ __forceinline__ float roulette_survivor(float w)
     {
         return (float)((double)w / 0.1);
     }
     static __device__ __forceinline__ float zero_threshold() { return (float)(1 - 0.99999); }
+    /* Whether a step needs the work that few do (photon_step).  One chain of compares,
+     * each taking the result so far: written in C the terms are combined by predicate
+     * instructions of their own (8.6 of the step's 192, 5.2 of 188 this way). */
+    static __device__ __forceinline__ bool rare(uint32_t changed, float W, float mu_t, float uz,
+                                                float least_u, float x, float Lx, float y, float Ly)
+    {
+        uint32_t any;
+        asm("{\n\t.reg .pred p;\n\t"
+            "setp.ne.u32 p, %1, 0;\n\t"
+            "setp.leu.or.f32 p, %2, %3, p;\n\t"
+            "setp.eq.or.f32 p, %4, 0f00000000, p;\n\t"
+            "setp.gtu.or.f32 p, %5, %6, p;\n\t"
+            "setp.lt.or.f32 p, %7, %8, p;\n\t"
+            "setp.leu.or.f32 p, %9, 0f00000000, p;\n\t"
+            "setp.geu.or.f32 p, %9, %10, p;\n\t"
+            "setp.leu.or.f32 p, %11, 0f00000000, p;\n\t"
+            "setp.geu.or.f32 p, %11, %12, p;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(any)
+            : "r"(changed), "f"(W), "f"(0x1.a36e2ep-14f), "f"(mu_t), "f"(fabsf(uz)),
+              "f"(0x1.fffeb0p-1f), "f"(least_u), "f"(zero_threshold()), "f"(x), "f"(Lx), "f"(y),
+              "f"(Ly));
+        return any != 0;
+    }
     /* fixed-point weight, 2^-32 resolution */
     static __device__ __forceinline__ uint64_t qw(float w) { return __float2ull_rn(w * 4294967296.0f); }
 };
 
 struct MathExact : FloatTable {
     static constexpr bool kFast = false;
+    using Pairs = PairwiseOps<MathExact, float>;
     static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
     static __device__ __forceinline__ float mad(float a, float b, float c) { return a * b + c; }
     static __device__ __forceinline__ float div(float a, float b) { return a / b; }
@@ -107,6 +207,7 @@ struct MathExact : FloatTable {
  * operators and functions below map to the approximate hardware paths. */
 struct MathFast : FloatTable {
     static constexpr bool kFast = true;
+    using Pairs = PackedOps;
     static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
     static __device__ __forceinline__ float mad(float a, float b, float c) { return __fmaf_rn(a, b, c); }
     /* every denominator divided here is a direction cosine, a sum of products of
@@ -147,6 +248,7 @@ struct MathFast : FloatTable {
 struct MathF64 {
     using real = double;
     static constexpr bool kFast = false;
+    using Pairs = PairwiseOps<MathF64, double>;
     static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
     static __device__ __forceinline__ double mad(double a, double b, double c) { return a * b + c; }
     static __device__ __forceinline__ double div(double a, double b) { return a / b; }
@@ -191,6 +293,13 @@ struct MathF64 {
     static __device__ __forceinline__ bool uz_within(double u) { return u <= 0.99999; }
     static __device__ __forceinline__ double roulette_survivor(double w) { return w / 0.1; }
     static __device__ __forceinline__ double zero_threshold() { return 1 - 0.99999; }
+    static __device__ __forceinline__ bool rare(uint32_t changed, double W, double mu_t, double uz,
+                                                double least_u, double x, double Lx, double y,
+                                                double Ly)
+    {
+        return changed | !w_above_threshold(W) | (mu_t == 0) | !uz_within(fabs(uz)) |
+               (least_u < zero_threshold()) | !(x > 0) | !(x < Lx) | !(y > 0) | !(y < Ly);
+    }
     static __device__ __forceinline__ uint64_t qw(double w)
     {
         return __double2ull_rn(w * 4294967296.0);
@@ -242,6 +351,22 @@ static __device__ __forceinline__ R grid_index(R x, R up, float d_, float rd_)
     return M::mad(on_face, M::mad((R)2, up, (R)-1), fi) - below;
 }
 
+/* grid_index of the x and y axes */
+template <class M, class R = typename M::real>
+static __device__ __forceinline__ Pair<R> grid_index2(Pair<R> x, Pair<R> up, const GeomDev &g)
+{
+    using Two = typename M::Pairs;
+    using P2 = Pair<R>;
+    const P2 d = {(R)g.dx, (R)g.dy};
+    const P2 q = Two::div_r(x, d, P2{(R)g.rdx, (R)g.rdy});
+    const P2 f = {M::floor(q.a), M::floor(q.b)};
+    const P2 face = Two::mul(Two::add(f, up), d), lo = Two::mul(f, d);
+    const P2 on_face = {x.a == face.a ? (R)1 : (R)0, x.b == face.b ? (R)1 : (R)0};
+    const P2 below = {x.a >= lo.a ? (R)0 : (R)1, x.b >= lo.b ? (R)0 : (R)1};
+    const P2 way = Two::mad(P2{(R)2, (R)2}, up, P2{(R)-1, (R)-1});
+    return Two::sub(Two::mad(on_face, way, f), below);
+}
+
 /* A voxel index as an int, before the clamp into the grid.  The conversion's own
  * result for the NaN position of a photon that the quickfix is about to remove (0
  * in FP32, below the range in FP64) less the face rule's one picks the first
@@ -267,7 +392,7 @@ static __device__ __forceinline__ int tissue_at(const GeomDev &g, R fi, R fj, R 
     } else {
         t = __ldg(g.tissue + ((int64_t)ck * g.ny + cj) * g.nx + ci);
     }
-    return ((z <= 0) && (uz < 0)) ? MC3D_TISSUE_AIR : t;
+    return ((z <= 0) & (uz < 0)) ? MC3D_TISSUE_AIR : t;
 }
 
 /* Distance to one face of the step's box along an axis (src/mc3d_gpu.cu:29-49): the
@@ -281,6 +406,19 @@ static __device__ __forceinline__ R face_distance(R x, R u, R up, R fi, R r, flo
     /* fi + r + 1 upward, fi - r downward (whole numbers: exact) */
     *border = M::mul(fi + M::mad(up, M::mad((R)2, r, (R)1), -r), (R)d);
     return M::div(*border - x, u);
+}
+
+/* face_distance of the x and y axes */
+template <class M, class R = typename M::real>
+static __device__ __forceinline__ Pair<R> face_distance2(Pair<R> x, Pair<R> u, Pair<R> up,
+                                                         Pair<R> fi, R r, const GeomDev &g,
+                                                         Pair<R> *border)
+{
+    using Two = typename M::Pairs;
+    const R span = M::mad((R)2, r, (R)1);
+    const Pair<R> off = {M::mad(up.a, span, -r), M::mad(up.b, span, -r)};
+    *border = Two::mul(Two::add(fi, off), Pair<R>{(R)g.dx, (R)g.dy});
+    return Two::div(Two::sub(*border, x), u);
 }
 
 /* src/mc3d_gpu.cu:113-126 */
@@ -302,7 +440,7 @@ struct PhotonT {
     int tissue;
 };
 
-/* Per-thread tallies live in shared memory, one column per thread, so that the
+/* Per-thread tallies live in shared memory, one row per thread, so that the
  * step loop keeps only the photon in registers.  They are touched when a photon
  * ends or at a roulette event, and flushed to the job's totals when the thread
  * moves to another stream.  Slot order is mc3d_totals (include/mc3d.h). */
@@ -310,15 +448,45 @@ enum {
     T_PHOTONS = 0, T_STEPS, T_W_LAUNCHED, T_R_IN, T_R_OUT, T_T_IN, T_T_OUT, T_ABSORBED,
     T_RR_KILLED, T_RR_CREATED, T_LOST, T_CAPPED, T_QUICKFIX, T_FRESNEL
 };
-#define MC3D_MAX_BLOCK 256
 
 struct Acc {
-    unsigned long long *col; /* sh_acc + threadIdx.x; slot t at col[t * MC3D_MAX_BLOCK] */
-    __device__ __forceinline__ unsigned long long &operator[](int t) const
-    {
-        return col[t * MC3D_MAX_BLOCK];
-    }
+    unsigned long long *row; /* the thread's MC3D_THREAD_WORDS words of shared memory */
+    __device__ __forceinline__ unsigned long long &operator[](int t) const { return row[t]; }
+    /* of the thread's stream: photons left and job-local index */
+    __device__ __forceinline__ int64_t &left() const { return (int64_t &)row[MC3D_NUM_TOTALS]; }
+    __device__ __forceinline__ int64_t &local() const { return (int64_t &)row[MC3D_NUM_TOTALS + 1]; }
 };
+
+/* Henyey-Greenstein scattering of the direction of p, src/mc3d_gpu.cu:282-294, by the
+ * draws e_hg (cosine) and e_phi (azimuth): the direction by the general formula, and
+ * the angles for the one along the z axis. */
+template <class R>
+struct Spin {
+    R ux, uy, uz, costheta, sintheta, cosphi, sinphi;
+};
+
+template <class M, bool SPLIT_SIN2, class R = typename M::real>
+static __device__ __forceinline__ Spin<R> scatter(const float4 *tt, const PhotonT<R> &p,
+                                                  uint32_t e_hg, uint32_t e_phi)
+{
+    Spin<R> o;
+    const R xi = (R)(1.0f - mc3d_u32_to_float_rz(e_hg) * 0x1p-32f);
+    o.costheta = M::template hg_cos<M>(tt, xi);
+    /* 1 - cos^2 with one rounding, but with two in the fast merged-step kernel that maps
+     * one geometry's absorption: that kernel has always rounded the square by itself, and
+     * a seeded run repeats its tallies */
+    o.sintheta = M::sqrt(SPLIT_SIN2 ? (R)1 - M::mul(o.costheta, o.costheta)
+                                    : M::mad(-o.costheta, o.costheta, (R)1));
+    M::sincos_draw(e_phi, &o.sinphi, &o.cosphi);
+    const R sin2 = M::mad(-p.uz, p.uz, (R)1);
+    const R invsqrt = M::rsqrt(sin2);
+    const R Ax = M::mad(-p.uy, o.sinphi, M::mul(M::mul(p.ux, p.uz), o.cosphi));
+    const R Ay = M::mad(p.ux, o.sinphi, M::mul(M::mul(p.uy, p.uz), o.cosphi));
+    o.ux = M::mad(p.ux, o.costheta, M::mul(M::mul(o.sintheta, Ax), invsqrt));
+    o.uy = M::mad(p.uy, o.costheta, M::mul(M::mul(o.sintheta, Ay), invsqrt));
+    o.uz = M::mad(p.uz, o.costheta, M::mul(M::mul(-M::sqrt(sin2), o.sintheta), o.cosphi));
+    return o;
+}
 
 /* One step of src/mc3d_gpu.cu:175-340 for a live photon.  Returns true when the
  * photon froze during this step; *db receives the step's boundary distance.
@@ -348,19 +516,21 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
                                                    const Acc &acc, R *db_out,
                                                    unsigned long long *amap, bool *lat_mirror)
 {
-    /* per tissue: (mua, mus, g, n), (mu_t, mua/mu_t, 1/mu_t, 1/(2g)),
+    /* per tissue: (mua, mus, g, n), (mu_t, 1/mu_t, mua/mu_t, 1/(2g)),
      * (1-g^2, 1-g, 2g, 1+g^2) -- each the float the reference computes per step */
     const float4 *tt = tab + MC3D_TAB_STRIDE * (JUMP ? (p.tissue & 0xff) : p.tissue);
     const R mu_t = M::mu_t(tt);
 
     /* the box's nearest face, src/mc3d_gpu.cu:29-49 */
     const R r = JUMP ? (R)(p.tissue >> 8) : (R)0;
-    R bx, by, bz;
-    const R up_x = upward(p.ux), up_y = upward(p.uy), up_z = upward(p.uz);
-    const R t_x = face_distance<M>(p.x, p.ux, up_x, p.i, r, g.dx, &bx);
-    const R t_y = face_distance<M>(p.y, p.uy, up_y, p.j, r, g.dy, &by);
+    using P2 = Pair<R>;
+    const P2 up = {upward(p.ux), upward(p.uy)};
+    const R up_z = upward(p.uz);
+    P2 bxy;
+    R bz;
+    const P2 t_xy = face_distance2<M>({p.x, p.y}, {p.ux, p.uy}, up, {p.i, p.j}, r, g, &bxy);
     const R t_z = face_distance<M>(p.z, p.uz, up_z, p.k, r, g.dz, &bz);
-    const R db = M::fmin(t_x, M::fmin(t_y, t_z));
+    const R db = M::fmin(t_xy.a, M::fmin(t_xy.b, t_z));
     *db_out = db;
 
     /* move to that face or to the interaction, whichever is nearer: one expression
@@ -372,25 +542,62 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
     R newx = M::advance(p.x, M::mul(p.ux, m), hit, db, mu_t, rmu_t);
     R newy = M::advance(p.y, M::mul(p.uy, m), hit, db, mu_t, rmu_t);
     R newz = M::advance(p.z, M::mul(p.uz, m), hit, db, mu_t, rmu_t);
-    newx = (hit && db == t_x) ? bx : newx;
-    newy = (hit && db == t_y) ? by : newy;
-    newz = (hit && db == t_z) ? bz : newz;
+    const R face = hit ? db : (R)__int_as_float(0x7fc00000); /* NaN: no face */
+    newx = (face == t_xy.a) ? bxy.a : newx;
+    newy = (face == t_xy.b) ? bxy.b : newy;
+    newz = (face == t_z) ? bz : newz;
     const R s = p.s - ds; /* what a hit leaves of the free path */
 
-    R nexti = grid_index<M>(newx, up_x, g.dx, g.rdx);
-    R nextj = grid_index<M>(newy, up_y, g.dy, g.rdy);
+    const P2 nextij = grid_index2<M>(P2{newx, newy}, up, g);
+    R nexti = nextij.a, nextj = nextij.b;
     R nextk = grid_index<M>(newz, up_z, g.dz, g.rdz);
     int next_tissue = tissue_at<JUMP>(g, nexti, nextj, nextk, newz, p.uz);
 
-    /* Fresnel, src/mc3d_gpu.cu:226-257.  The index is looked up only where the
-     * tissue changes.  A photon that goes on from a face (hit) takes the new
-     * direction here; without a hit the direction is the scattered one below, and
-     * a frozen photon keeps its own. */
-    bool refl = false;
-    if (JUMP ? ((next_tissue ^ p.tissue) & 0xff) != 0 : next_tissue != p.tissue) {
+    /* the step's draws: roulette, scattering cosine and azimuth, next free path */
+    rx = mc3d_mwc_next(rx, ra);
+    uint32_t e_rr = (uint32_t)rx;
+    rx = mc3d_mwc_next(rx, ra);
+    uint32_t e_hg = (uint32_t)rx;
+    rx = mc3d_mwc_next(rx, ra);
+    uint32_t e_phi = (uint32_t)rx;
+    rx = mc3d_mwc_next(rx, ra);
+    uint32_t e_s = (uint32_t)rx;
+
+    /* absorption, src/mc3d_gpu.cu:262-263 */
+    R W = p.W - (hit ? (R)0 : M::mul(M::albedo_c(tt), p.W));
+    if (AMAP && !hit && mu_t > 0) {
+        /* absorption map, the reference's disabled tally (src/mc3d_gpu.cu:265-272):
+         * the current voxel clamped into the grid, fixed-point weight removed.  A
+         * merged step can end its flight several voxels from where it started, so
+         * there the voxel of the interaction point is used. */
+        const int ai = min(max((int)(JUMP ? nexti : p.i), 0), g.nx - 1);
+        const int aj = min(max((int)(JUMP ? nextj : p.j), 0), g.ny - 1);
+        const int ak = min(max((int)(JUMP ? nextk : p.k), 0), g.nz - 1);
+        const uint64_t dq = M::qw(p.W) - M::qw(W);
+        if (dq) atomicAdd(amap + ((int64_t)ak * g.ny + aj) * g.nx + ai, (unsigned long long)dq);
+    }
+
+    /* the scattered direction, or for a hit the old one */
+    R nux = p.ux, nuy = p.uy, nuz = p.uz;
+    const Spin<R> spin = scatter<M, SPLIT_SIN2>(tt, p, e_hg, e_phi);
+    nux = (!hit) ? spin.ux : nux;
+    nuy = (!hit) ? spin.uy : nuy;
+    nuz = (!hit) ? spin.uz : nuz;
+
+    /* What few steps need, behind one test: another tissue, a weight below the
+     * roulette's threshold, air, components that snap to zero, the scattering of a
+     * photon along the z axis, and the lateral faces.  The cell is looked up above
+     * and first looked at here, so the scattering hides the load. */
+    const R zero_thresh = M::zero_threshold();
+    const bool steep = !M::uz_within(M::fabs(p.uz));
+    const uint32_t changed = (uint32_t)(next_tissue ^ p.tissue) & 0xffu;
+    if (M::rare(changed, W, mu_t, p.uz, M::fmin(M::fabs(nux), M::fmin(M::fabs(nuy), M::fabs(nuz))),
+                newx, g.Lx, newy, g.Ly)) {
+        bool refl = false;
+        bool again = steep && !hit;
         const R ni = M::n(tt);
         const R nt = M::n(tab + MC3D_TAB_STRIDE * (JUMP ? (next_tissue & 0xff) : next_tissue));
-        if (ni != nt) {
+        if (ni != nt) { /* Fresnel, src/mc3d_gpu.cu:226-257 */
             const bool mx = p.i != nexti, my = p.j != nextj, mz = p.k != nextk;
             R cos_ai = mx ? p.ux : (my ? p.uy : p.uz);
             cos_ai = M::fabs(cos_ai);
@@ -432,56 +639,28 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
                 cos_at = (R)(ca * sc);
                 lat = (R)(rn * sc);
             }
-            const float eps = mc3d_rand_co(&rx, ra);
-            refl = eps < Rf;
-            if (hit && mu_t != 0 && !(p.W <= 0)) {
+            /* The reflection is the step's first draw, so the other four are each one
+             * draw later than taken above. */
+            refl = mc3d_u32_to_float_rz(e_rr) * 0x1p-32f < Rf;
+            e_rr = e_hg;
+            e_hg = e_phi;
+            e_phi = e_s;
+            rx = mc3d_mwc_next(rx, ra);
+            e_s = (uint32_t)rx;
+            if (hit) {
                 const R tx = mx ? M::copysign(cos_at, M::mul(p.ux, cos_at)) : M::mul(p.ux, lat);
                 const R ty = (my && !mx) ? M::copysign(cos_at, M::mul(p.uy, cos_at))
                                          : M::mul(p.uy, lat);
                 const R tz = (mz && !my && !mx) ? M::copysign(cos_at, M::mul(p.uz, cos_at))
                                                 : M::mul(p.uz, lat);
-                p.ux = refl ? (mx ? -p.ux : p.ux) : tx;
-                p.uy = refl ? (my ? -p.uy : p.uy) : ty;
-                p.uz = refl ? (mz ? -p.uz : p.uz) : tz;
+                nux = refl ? (mx ? -p.ux : p.ux) : tx;
+                nuy = refl ? (my ? -p.uy : p.uy) : ty;
+                nuz = refl ? (mz ? -p.uz : p.uz) : tz;
             }
-            if (hit && refl) { /* a reflected photon keeps its voxel (:334-339) */
-                nexti = p.i;
-                nextj = p.j;
-                nextk = p.k;
-                next_tissue = p.tissue;
-            }
+            again = !hit; /* an interaction that rounded onto the face */
             acc[T_FRESNEL] += 1;
         }
-    }
-
-    /* the step's draws: roulette, scattering cosine and azimuth, next free path */
-    rx = mc3d_mwc_next(rx, ra);
-    const uint32_t e_rr = (uint32_t)rx;
-    rx = mc3d_mwc_next(rx, ra);
-    const uint32_t e_hg = (uint32_t)rx;
-    rx = mc3d_mwc_next(rx, ra);
-    const uint32_t e_phi = (uint32_t)rx;
-    rx = mc3d_mwc_next(rx, ra);
-    uint32_t e_s = (uint32_t)rx;
-
-    /* absorption, src/mc3d_gpu.cu:262-263 */
-    R W = p.W;
-    W = W - (hit ? (R)0 : M::mul(M::albedo_c(tt), W));
-    if (AMAP && !hit && mu_t > 0) {
-        /* absorption map, the reference's disabled tally (src/mc3d_gpu.cu:265-272):
-         * the current voxel clamped into the grid, fixed-point weight removed.  A
-         * merged step can end its flight several voxels from where it started, so
-         * there the voxel of the interaction point is used. */
-        const int ai = min(max((int)(JUMP ? nexti : p.i), 0), g.nx - 1);
-        const int aj = min(max((int)(JUMP ? nextj : p.j), 0), g.ny - 1);
-        const int ak = min(max((int)(JUMP ? nextk : p.k), 0), g.nz - 1);
-        const uint64_t dq = M::qw(p.W) - M::qw(W);
-        if (dq) atomicAdd(amap + ((int64_t)ak * g.ny + aj) * g.nx + ai, (unsigned long long)dq);
-    }
-
-    /* Russian roulette (src/mc3d_gpu.cu:275-277) and freezing (:303-311), both
-     * behind the one rare test that either needs */
-    if (!M::w_above_threshold(W) || mu_t == 0) {
+        /* Russian roulette, src/mc3d_gpu.cu:275-277 */
         if (M::w_below_threshold(W) && !hit && mu_t != 0) {
             const float eps = mc3d_u32_to_float_rz(e_rr) * 0x1p-32f;
             const R newW = (eps < MC3D_SURVIVAL_LT_F) ? M::roulette_survivor(W) : (R)0;
@@ -498,7 +677,7 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
             }
             W = newW;
         }
-        if (W <= 0 || mu_t == 0) { /* freeze: the photon stays where it is */
+        if (W <= 0 || mu_t == 0) { /* freeze (:303-311): the photon stays where it is */
             p.W = W;
             p.s = hit ? s : p.s - p.s;
             *lat_mirror = false;
@@ -507,48 +686,20 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
             return true;
         }
         if (!(W > 0)) e_s = 0; /* NaN weight: no free path, -log(1) */
-    }
-    p.W = W;
-
-    /* Henyey-Greenstein, src/mc3d_gpu.cu:282-294 */
-    const R xi = (R)(1.0f - mc3d_u32_to_float_rz(e_hg) * 0x1p-32f);
-    const R costheta = M::template hg_cos<M>(tt, xi);
-    /* 1 - cos^2 with one rounding, but with two in the fast merged-step kernel that maps
-     * one geometry's absorption: that kernel has always rounded the square by itself, and
-     * a seeded run repeats its tallies */
-    const R sintheta = M::sqrt(SPLIT_SIN2 ? (R)1 - M::mul(costheta, costheta)
-                                          : M::mad(-costheta, costheta, (R)1));
-    R cosphi, sinphi;
-    M::sincos_draw(e_phi, &sinphi, &cosphi);
-    const R sin2 = M::mad(-p.uz, p.uz, (R)1);
-    const R invsqrt = M::rsqrt(sin2);
-    const R Ax = M::mad(-p.uy, sinphi, M::mul(M::mul(p.ux, p.uz), cosphi));
-    const R Ay = M::mad(p.ux, sinphi, M::mul(M::mul(p.uy, p.uz), cosphi));
-    const R sc_ux = M::mad(p.ux, costheta, M::mul(M::mul(sintheta, Ax), invsqrt));
-    const R sc_uy = M::mad(p.uy, costheta, M::mul(M::mul(sintheta, Ay), invsqrt));
-    const R sc_uz = M::mad(p.uz, costheta, M::mul(M::mul(-M::sqrt(sin2), sintheta), cosphi));
-    R nux = (!hit) ? sc_ux : p.ux;
-    R nuy = (!hit) ? sc_uy : p.uy;
-    R nuz = (!hit) ? sc_uz : p.uz;
-
-    /* What few steps need, behind one test: the scattering of a photon along the z
-     * axis, components snapped to zero, and the mirrors at the lateral faces
-     * (short-circuited as in src/mc3d_gpu.cu:330), which are no-ops off them.  A
-     * mirror turns its component before the normalisation, which keeps the sign. */
-    const R zero_thresh = M::zero_threshold();
-    const bool steep = !M::uz_within(M::fabs(p.uz));
-    if (steep || M::fabs(nux) < zero_thresh || M::fabs(nuy) < zero_thresh ||
-        M::fabs(nuz) < zero_thresh || !(newx > 0 && newx < g.Lx && newy > 0 && newy < g.Ly)) {
-        if (steep && !hit) {
-            nux = M::mul(sintheta, cosphi);
-            nuy = M::mul(sintheta, sinphi);
-            nuz = M::copysign(costheta, M::mul(costheta, p.uz));
+        if (again) {
+            const Spin<R> sp = scatter<M, SPLIT_SIN2>(tt, p, e_hg, e_phi);
+            nux = steep ? M::mul(sp.sintheta, sp.cosphi) : sp.ux;
+            nuy = steep ? M::mul(sp.sintheta, sp.sinphi) : sp.uy;
+            nuz = steep ? M::copysign(sp.costheta, M::mul(sp.costheta, p.uz)) : sp.uz;
         }
         nux = (M::fabs(nux) < zero_thresh) ? 0 : nux;
         nuy = (M::fabs(nuy) < zero_thresh) ? 0 : nuy;
         nuz = (M::fabs(nuz) < zero_thresh) ? 0 : nuz;
-        if (!refl && (mirror<M>(&newx, &nux, g.Lx) || mirror<M>(&newy, &nuy, g.Ly)) && hit) {
-            nexti = p.i; /* as after a Fresnel reflection */
+        /* mirrors, short-circuited as in src/mc3d_gpu.cu:330.  A mirror turns its
+         * component before the normalisation, which keeps the sign. */
+        refl = refl || mirror<M>(&newx, &nux, g.Lx) || mirror<M>(&newy, &nuy, g.Ly);
+        if (hit && refl) { /* a reflected photon keeps its voxel (:334-339) */
+            nexti = p.i;
             nextj = p.j;
             nextk = p.k;
             next_tissue = p.tissue;
@@ -561,6 +712,7 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
 
     const R newS = -M::log((R)(1.0f - mc3d_u32_to_float_rz(e_s) * 0x1p-32f));
     p.s = hit ? s : newS;
+    p.W = W;
     p.x = newx;
     p.y = newy;
     p.z = newz;
@@ -715,40 +867,49 @@ template <class M, bool AMAP, bool JUMP = false, bool ONE_GEOM = false>
 __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
 {
     using R = typename M::real;
-    /* dynamic shared memory: the optical tables, then (several geometries) the
-     * geometry descriptors, read from there instead of being held per thread */
-    extern __shared__ float4 sh_tab[];
-    __shared__ unsigned long long sh_acc[MC3D_NUM_TOTALS * MC3D_MAX_BLOCK];
+    /* dynamic shared memory (photon_smem): the threads' rows, then the optical tables,
+     * then (several geometries) the geometry descriptors, read from there instead of
+     * being held per thread.  Sized by the block, so the rest stays with the L1 cache,
+     * which holds cells. */
+    extern __shared__ float4 sh_base[];
+    unsigned long long *sh_rows = reinterpret_cast<unsigned long long *>(sh_base);
+    float4 *sh_tab = reinterpret_cast<float4 *>(sh_rows + MC3D_THREAD_WORDS * blockDim.x);
     for (int t = threadIdx.x; t < P.props_entries; t += blockDim.x) sh_tab[t] = P.props_table[t];
     GeomDev *sh_geom = reinterpret_cast<GeomDev *>(sh_tab + P.props_entries);
     if (!ONE_GEOM)
         for (int t = threadIdx.x; t < P.ngeoms; t += blockDim.x) sh_geom[t] = P.geoms[t];
-    const Acc acc{sh_acc + threadIdx.x};
+    const Acc acc{sh_rows + MC3D_THREAD_WORDS * threadIdx.x};
     acc_clear(acc);
     __syncthreads();
 
     int job = -1;
     const GeomDev *gp = sh_geom;
     const float4 *tab = sh_tab;
-    int64_t left = 0, local = 0;
+    int64_t &left = acc.left(), &local = acc.local();
+    left = 0;
     uint64_t rx = 0;
     uint32_t ra = 1;
     PhotonT<R> p;
     bool alive = false;
+    bool drained = false; /* no stream left to take */
     int psteps = 0; /* steps of the photon before its present chunk */
     unsigned long long *amap = nullptr;
 
     /* One iteration is one 45-step chunk, the reference's launch.  A photon starts
      * only at a chunk's start, as a reference slot starts only at a launch boundary:
      * a lane whose photon ended waits out the rest of the chunk (the reference's
-     * masked steps), so the lanes of a warp start, end and refill photons together
-     * and the step loop itself holds nothing but steps. */
+     * masked steps).  The two warp barriers make that wait real: without them a lane
+     * that leaves the step loop early runs on alone, and from then on the warp steps
+     * in pieces (22.5 lanes a step and 4.7 a chunk's end instead of 30 and 30, layered
+     * 1e6 photons).  Lanes without a photon stay in the loop until the warp has none. */
     for (;;) {
-        if (!alive) {
+        if (!alive && !drained) {
             while (left == 0) {
-                if (P.cancel && *((volatile const int *)P.cancel)) break;
+                drained = P.cancel && *((volatile const int *)P.cancel);
+                if (drained) break;
                 int64_t gs = (int64_t)atomicAdd((unsigned long long *)P.work_counter, 1ull);
-                if (gs >= P.total_streams) break;
+                drained = gs >= P.total_streams;
+                if (drained) break;
                 const int next_job = find_job(P.jobs, P.njobs, gs);
                 /* the per-thread tallies are the job's: flushed when the job changes */
                 if (job >= 0 && next_job != job)
@@ -763,7 +924,8 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
                 ra = stream_multiplier(P, local);
                 rx = stream_seed(P, jb, local, ra);
             }
-            if (left == 0) break;
+        }
+        if (!alive && !drained) {
             const GeomDev &g = ONE_GEOM ? P.geom0 : *gp;
             /* photontrack_reinitialize, src/mc3d_gpu.cu:74-111 */
             if (P.jobs[job].beam == 0) {
@@ -786,6 +948,7 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
             alive = true;
             left--;
         }
+        if (!__any_sync(0xffffffffu, alive)) break;
 
         const GeomDev &g = ONE_GEOM ? P.geom0 : *gp;
         /* The chunk's steps, fewer where the step cap comes first.  Merged steps: the
@@ -794,23 +957,25 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
          * uniform cube), or merged steps would lose less weight to it than the
          * reference does.  It is taken from that step's start state, so the loop
          * stops before that step and goes round once more for it. */
-        const int cap = min(MC3D_NUM_PHOTON_STEPS, (int)P.max_steps - psteps);
+        const int cap = alive ? min(MC3D_NUM_PHOTON_STEPS, (int)P.max_steps - psteps) : 0;
         int stop = JUMP ? min(cap, MC3D_NUM_PHOTON_STEPS - 1) : cap;
         int chunk = 0;
         R db;
         bool lat_mirror;
-        bool froze;
+        bool froze = false;
         bool vzero = false;
         for (;;) {
-            do {
+            while (!froze && chunk < stop) {
                 froze = photon_step<M, AMAP, JUMP, M::kFast && AMAP && JUMP && ONE_GEOM>(
                     g, tab, p, rx, ra, acc, &db, amap, &lat_mirror);
                 chunk++;
-            } while (!froze && chunk < stop);
+            }
             if (!JUMP || froze || stop == cap) break;
             vzero = voxel_db<M>(g, p) == 0;
             stop = cap;
         }
+        __syncwarp();
+        if (!alive) continue;
         psteps += chunk;
 
         bool done = false;

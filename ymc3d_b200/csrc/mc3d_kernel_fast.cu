@@ -8,56 +8,61 @@
 
 namespace mc3d {
 
-/* Eight instantiations: merged steps (box DDA over uniform cubes) or one step
+/* 96 registers: 20 warps an SM in blocks of 128 threads, and no spills.  80 registers
+ * (24 warps) spill 120 bytes a step, 104 (16 warps) hide less: 1e7 layered photons took
+ * 174.4 ms with 80, 175.5 with 96 and 184.5 with 104, 2e5 skin-model photons 4.59, 3.97
+ * and 3.59 ms, because a photon's own steps come slower the more warps share an SM.
+ *
+ * Eight instantiations: merged steps (box DDA over uniform cubes) or one step
  * per voxel face; with or without the absorption map; several geometries (their
  * descriptors in shared memory) or one (its descriptor read from the kernel
  * parameters, which keeps it out of the registers). */
 
 /* merged steps */
-__global__ void __launch_bounds__(256, 3) photon_kernel_fast(const __grid_constant__ KernelParams P)
+__global__ void __maxnreg__(96) photon_kernel_fast(const __grid_constant__ KernelParams P)
 {
     photon_kernel_body<MathFast, false, true>(P);
 }
 
 /* merged steps with the per-voxel absorption map */
-__global__ void __launch_bounds__(256, 3)
+__global__ void __maxnreg__(96)
     photon_kernel_fast_amap(const __grid_constant__ KernelParams P)
 {
     photon_kernel_body<MathFast, true, true>(P);
 }
 
 /* one step per voxel face, as the reference steps */
-__global__ void __launch_bounds__(256, 3)
+__global__ void __maxnreg__(96)
     photon_kernel_fast_voxel(const __grid_constant__ KernelParams P)
 {
     photon_kernel_body<MathFast, false, false>(P);
 }
 
-__global__ void __launch_bounds__(256, 3)
+__global__ void __maxnreg__(96)
     photon_kernel_fast_voxel_amap(const __grid_constant__ KernelParams P)
 {
     photon_kernel_body<MathFast, true, false>(P);
 }
 
 /* one geometry */
-__global__ void __launch_bounds__(256, 3) photon_kernel_fast_g1(const __grid_constant__ KernelParams P)
+__global__ void __maxnreg__(96) photon_kernel_fast_g1(const __grid_constant__ KernelParams P)
 {
     photon_kernel_body<MathFast, false, true, true>(P);
 }
 
-__global__ void __launch_bounds__(256, 3)
+__global__ void __maxnreg__(96)
     photon_kernel_fast_amap_g1(const __grid_constant__ KernelParams P)
 {
     photon_kernel_body<MathFast, true, true, true>(P);
 }
 
-__global__ void __launch_bounds__(256, 3)
+__global__ void __maxnreg__(96)
     photon_kernel_fast_voxel_g1(const __grid_constant__ KernelParams P)
 {
     photon_kernel_body<MathFast, false, false, true>(P);
 }
 
-__global__ void __launch_bounds__(256, 3)
+__global__ void __maxnreg__(96)
     photon_kernel_fast_voxel_amap_g1(const __grid_constant__ KernelParams P)
 {
     photon_kernel_body<MathFast, true, false, true>(P);

@@ -18,6 +18,15 @@ namespace mc3d {
 #define MC3D_VARIANT_VOXEL_STEPS 2
 /* one geometry in the launch: its descriptor is read from the kernel parameters */
 #define MC3D_VARIANT_ONE_GEOM 4
+
+/* dynamic shared memory of a photon kernel: the threads' rows, optical tables, geometry
+ * descriptors */
+static inline size_t photon_smem(int props_entries, int ngeoms, int block)
+{
+    return sizeof(unsigned long long) * MC3D_THREAD_WORDS * (size_t)block +
+           sizeof(float4) * (size_t)props_entries + sizeof(GeomDev) * (size_t)ngeoms;
+}
+
 cudaError_t launch_photon_fast(const KernelParams &P, int grid, int block, size_t smem,
                                cudaStream_t stream, int variant);
 cudaError_t launch_photon_exact(const KernelParams &P, int grid, int block, size_t smem,

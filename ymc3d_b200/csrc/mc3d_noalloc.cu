@@ -66,7 +66,7 @@ static_assert(sizeof(JobDev) <= 256 && sizeof(GeomDev) <= 256, "descriptor slots
 static __device__ __align__(256) unsigned char g_noalloc_scratch[MC3D_NOALLOC_SCRATCH_BYTES];
 
 /* one geometry, per-face steps; the descriptor is read from P.geom0 */
-__global__ void __launch_bounds__(256, 3)
+__global__ void __maxnreg__(96)
     photon_kernel_noalloc(const __grid_constant__ KernelParams P)
 {
     photon_kernel_body<MathFast, false, false, true>(P);
@@ -181,7 +181,7 @@ extern "C" int mc3d_run_noalloc(const mc3d_geom *geom, const mc3d_props *props,
         volatile float frac = mut > 0 ? mua / mut : 0.0f, rmut = 1.0f / mut, g2 = g * g, twog = 2 * g;
         volatile float inv2g = 1.0f / twog;
         tab[3 * t + 0] = make_float4(mua, mus, g, props->n[t]);
-        tab[3 * t + 1] = make_float4(mut, frac, rmut, inv2g);
+        tab[3 * t + 1] = make_float4(mut, rmut, frac, inv2g);
         tab[3 * t + 2] = make_float4(1 - g2, 1 - g, twog, 1 + g2);
     }
     GeomDev gd;
@@ -272,10 +272,11 @@ extern "C" int mc3d_run_noalloc(const mc3d_geom *geom, const mc3d_props *props,
     P.seed = sc;
     int sms = 0, bps = 0;
     NA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    size_t smem = sizeof(float4) * P.props_entries;
-    NA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, photon_kernel_noalloc, 256, smem));
+    const int block = 128; /* at most 28 KB of shared memory: no opt-in */
+    size_t smem = photon_smem(P.props_entries, 0, block);
+    NA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, photon_kernel_noalloc, block, smem));
     if (bps <= 0) return nfail(MC3D_ERR_CAPACITY, "kernel does not fit an SM");
-    photon_kernel_noalloc<<<sms * bps, 256, smem, s>>>(P);
+    photon_kernel_noalloc<<<sms * bps, block, smem, s>>>(P);
     NA_TRY(cudaGetLastError());
     return MC3D_OK;
 }
