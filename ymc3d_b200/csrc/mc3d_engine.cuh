@@ -861,6 +861,20 @@ static __device__ __forceinline__ uint64_t stream_seed(const KernelParams &P, co
     return mc3d_seed_attempt(xs, P.seed.begin, fora);
 }
 
+/* A photon on its way from one thread of the block to another, in the tally words of
+ * the receiving thread's row (the stream's words go to their own place). */
+template <class R>
+struct ParkedT {
+    uint64_t rx;
+    R x, y, z, ux, uy, uz, W, s, i, j, k;
+    int32_t tissue;
+    uint32_t ra;
+    int32_t psteps, job;
+};
+static_assert(sizeof(ParkedT<double>) <= 8 * MC3D_NUM_TOTALS, "a photon outgrows the tally words");
+
+#define MC3D_MAX_WARPS 8 /* per block: 256 threads */
+
 /* The persistent photon loop.  JUMP selects merged steps (photon_step) and needs
  * every geometry's safe-distance map. */
 template <class M, bool AMAP, bool JUMP = false, bool ONE_GEOM = false>
@@ -880,6 +894,9 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
         for (int t = threadIdx.x; t < P.ngeoms; t += blockDim.x) sh_geom[t] = P.geoms[t];
     const Acc acc{sh_rows + MC3D_THREAD_WORDS * threadIdx.x};
     acc_clear(acc);
+    __shared__ volatile int sh_drain;          /* a thread found no stream left */
+    __shared__ int sh_live[2][MC3D_MAX_WARPS]; /* photons per warp, two chunks' worth */
+    if (threadIdx.x == 0) sh_drain = 0;
     __syncthreads();
 
     int job = -1;
@@ -894,6 +911,8 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
     bool drained = false; /* no stream left to take */
     int psteps = 0; /* steps of the photon before its present chunk */
     unsigned long long *amap = nullptr;
+    bool drain = false; /* the block is past the last stream */
+    int turn = 0;
 
     /* One iteration is one 45-step chunk, the reference's launch.  A photon starts
      * only at a chunk's start, as a reference slot starts only at a launch boundary:
@@ -948,7 +967,66 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
             alive = true;
             left--;
         }
-        if (!__any_sync(0xffffffffu, alive)) break;
+        /* The drain.  Once the streams run out, lanes fall idle one by one and the last
+         * photons of a launch, up to 15 times the mean length, would leave warps stepping
+         * for one or two lanes each and, by sharing an SM, slowing one another.  So from
+         * then on the block's warps meet at each chunk's start and, whenever its photons
+         * fit into fewer warps, close ranks: at most seven times, a photon's state passing
+         * through shared memory.  Where a photon is stepped changes nothing in its
+         * trajectory. */
+        if (!drain) {
+            if (drained) sh_drain = 1;
+            drain = __any_sync(0xffffffffu, sh_drain != 0);
+        }
+        if (drain) {
+            const unsigned live = __ballot_sync(0xffffffffu, alive);
+            int *count = sh_live[turn];
+            turn ^= 1; /* the other half is written only after all have read this one */
+            if ((threadIdx.x & 31) == 0) count[threadIdx.x >> 5] = __popc(live);
+            __syncthreads();
+            int total = 0, before = 0, warps = 0;
+            for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
+                if (w == (int)(threadIdx.x >> 5)) before = total;
+                total += count[w];
+                warps += count[w] != 0;
+            }
+            if (total == 0) break;
+            if ((total + 31) / 32 < warps) {
+                /* the rows become free of tallies, then carry the photons */
+                if (job >= 0) acc_flush(acc, P.totals + (int64_t)job * MC3D_NUM_TOTALS);
+                const int64_t my_left = left, my_local = local;
+                __syncthreads();
+                if (alive) {
+                    const int to = before + __popc(live & ((1u << (threadIdx.x & 31)) - 1u));
+                    const Acc other{sh_rows + MC3D_THREAD_WORDS * to};
+                    *reinterpret_cast<ParkedT<R> *>(other.row) = ParkedT<R>{
+                        rx, p.x, p.y, p.z, p.ux, p.uy, p.uz, p.W, p.s, p.i, p.j, p.k,
+                        p.tissue, ra, psteps, job};
+                    other.left() = my_left;
+                    other.local() = my_local;
+                }
+                __syncthreads();
+                alive = (int)threadIdx.x < total;
+                drained = !alive;
+                if (alive) {
+                    const ParkedT<R> q = *reinterpret_cast<const ParkedT<R> *>(acc.row);
+                    rx = q.rx;
+                    p.x = q.x; p.y = q.y; p.z = q.z;
+                    p.ux = q.ux; p.uy = q.uy; p.uz = q.uz;
+                    p.W = q.W; p.s = q.s;
+                    p.i = q.i; p.j = q.j; p.k = q.k;
+                    p.tissue = q.tissue;
+                    ra = q.ra;
+                    psteps = q.psteps;
+                    job = q.job;
+                    gp = sh_geom + P.jobs[job].geom;
+                    tab = sh_tab + P.jobs[job].props_offset;
+                    if (AMAP) amap = P.amap + P.jobs[job].amap_offset;
+                }
+                asm volatile("" ::: "memory"); /* the row is read before it is cleared */
+                acc_clear(acc);
+            }
+        }
 
         const GeomDev &g = ONE_GEOM ? P.geom0 : *gp;
         /* The chunk's steps, fewer where the step cap comes first.  Merged steps: the
