@@ -609,8 +609,8 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
                                       : M::sin(M::acos(cos_ai));
             const R sin_at = M::mul(ni_nt, sin_ai);
             R cos_at = M::sqrt(M::mad(-sin_at, sin_at, (R)1));
-            const R sc = M::mul(sin_ai, cos_at), cc = M::mul(cos_ai, cos_at);
-            const R R1 = M::div(M::mad(-cos_ai, sin_at, sc), M::mad(cos_ai, sin_at, sc));
+            const R cs = M::mul(cos_ai, sin_at), cc = M::mul(cos_ai, cos_at);
+            const R R1 = M::div(M::mad(sin_ai, cos_at, -cs), M::mad(sin_ai, cos_at, cs));
             const R R2 = M::div(M::mad(-sin_ai, sin_at, cc), M::mad(sin_at, sin_at, cc));
             /* 0.5 is a double literal there too */
             R Rf = 0.5 * R1 * R1 * M::mad(R2, R2, (R)1);
@@ -958,9 +958,8 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
             p.ux = 0; p.uy = 0; p.uz = 1;
             /* specular reflection from air into tissue type 1 (src/mc3d_gpu.cu:67-70, 500) */
             const R n0 = M::n(tab + MC3D_TAB_STRIDE * MC3D_TISSUE_AIR), n1 = M::n(tab + MC3D_TAB_STRIDE);
-            R rsp = M::div(n0 - n1, n0 + n1);
-            rsp = M::mul(rsp, rsp);
-            p.W = (R)1 - rsp;
+            const R rsp = M::div(n0 - n1, n0 + n1);
+            p.W = M::mad(-rsp, rsp, (R)1);
             p.s = -M::log((R)mc3d_rand_oc(&rx, ra));
             derive_cell<M, JUMP>(g, p);
             psteps = 0;
@@ -1117,9 +1116,8 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
             acc[slot] += q;
             /* the launch weight 1 - Rsp again, as at the photon's start */
             const R n0 = M::n(tab + MC3D_TAB_STRIDE * MC3D_TISSUE_AIR), n1 = M::n(tab + MC3D_TAB_STRIDE);
-            R rsp = M::div(n0 - n1, n0 + n1);
-            rsp = M::mul(rsp, rsp);
-            const uint64_t qw0 = M::qw((R)1 - rsp);
+            const R rsp = M::div(n0 - n1, n0 + n1);
+            const uint64_t qw0 = M::qw(M::mad(-rsp, rsp, (R)1));
             acc[T_W_LAUNCHED] += qw0;
             acc[T_ABSORBED] += qw0 - q - lost;
             acc[T_LOST] += lost;
