@@ -316,7 +316,7 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
         return fail(MC3D_ERR_ARG, "block must be a multiple of 32 up to 256, got %d", opt.block);
 
     /* ---- validate geometry and optical sets */
-    std::vector<int> max_tissue(ngeoms, 0);
+    std::vector<int> min_tissue(ngeoms, 0), max_tissue(ngeoms, 0);
     for (int i = 0; i < ngeoms; i++) {
         const mc3d_geom &g = geoms[i];
         if (g.nx <= 0 || g.ny <= 0 || g.nz <= 0 || !g.tissue)
@@ -325,8 +325,12 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
             !std::isfinite(g.dy) || !std::isfinite(g.dz))
             return fail(MC3D_ERR_GEOMETRY, "geometry %d: bad voxel size", i);
         int64_t nv = (int64_t)g.nx * g.ny * g.nz;
-        uint8_t mx = 0;
-        for (int64_t v = 0; v < nv; v++) mx = std::max(mx, g.tissue[v]);
+        uint8_t mn = 255, mx = 0;
+        for (int64_t v = 0; v < nv; v++) {
+            mn = std::min(mn, g.tissue[v]);
+            mx = std::max(mx, g.tissue[v]);
+        }
+        min_tissue[i] = mn;
         max_tissue[i] = mx;
     }
     std::vector<int> props_offset(nprops);
@@ -458,11 +462,9 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
         if ((uint64_t)geoms[i].nx * geoms[i].ny * ((uint64_t)geoms[i].nz + MC3D_SAFE_CAP) >=
             (1ull << 32))
             p->jump = false;
-    size_t max_map = 0; /* largest safe-distance map, nz + MC3D_SAFE_CAP slices */
     for (int i = 0; i < ngeoms; i++) {
         const mc3d_geom &g = geoms[i];
         size_t nv = (size_t)g.nx * g.ny * g.nz;
-        max_map = std::max(max_map, (size_t)g.nx * g.ny * (g.nz + MC3D_SAFE_CAP));
         PLAN_TRY(pool_alloc(&p->d_grids[i], nv, p->device, p->stream));
         PLAN_TRY(cudaMemcpyAsync(p->d_grids[i], g.tissue, nv, cudaMemcpyHostToDevice, p->stream));
         GeomDev &d = gh[i];
@@ -477,39 +479,45 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
         d.tissue = p->d_grids[i];
     }
     if (p->jump) {
-        /* per geometry: the safe-distance maps of the tissue grid and of its
-         * refractive-index classes, packed with the tissue into 16-bit cells
-         * (scratch: two pass buffers, the two maps and the class grid) */
+        /* per geometry: the safe distances of the tissue grid and of its
+         * refractive-index classes, packed with the tissue into 16-bit cells; the
+         * scratch is the largest geometry's */
         p->d_cells.assign(ngeoms, nullptr);
-        size_t max_vox = 0;
-        for (int i = 0; i < ngeoms; i++)
-            max_vox = std::max(max_vox, (size_t)geoms[i].nx * geoms[i].ny * geoms[i].nz);
+        struct Cells {
+            uint8_t classes[256];
+            bool shared, one_index;
+            int one_tissue;
+        };
+        std::vector<Cells> how(ngeoms);
+        size_t scratch = 0;
+        for (int i = 0; i < ngeoms; i++) {
+            const mc3d_geom &g = geoms[i];
+            Cells &c = how[i];
+            const int lo = min_tissue[i], hi = max_tissue[i];
+            c.one_tissue = lo == hi ? lo : -1;
+            c.shared = index_classes(i, hi, props, jobs, njobs, c.classes);
+            c.one_index = lo > 0;
+            for (int t = lo; t <= hi; t++) c.one_index &= c.classes[t] == c.classes[lo];
+            if (c.one_tissue < 0)
+                scratch = std::max(scratch, safe_distance_scratch(g.nx, g.ny, g.nz,
+                                                                  c.shared && !c.one_index));
+        }
         uint8_t *tmp = nullptr;
-        PLAN_TRY(pool_alloc(&tmp, 4 * max_map + max_vox, p->device, p->stream));
-        uint8_t *map_t = tmp + 2 * max_map, *map_n = tmp + 3 * max_map, *cls = tmp + 4 * max_map;
+        PLAN_TRY(pool_alloc(&tmp, scratch, p->device, p->stream));
         cudaError_t e = cudaSuccess;
         for (int i = 0; i < ngeoms && e == cudaSuccess; i++) {
             const mc3d_geom &g = geoms[i];
+            const Cells &c = how[i];
             size_t nmap = (size_t)g.nx * g.ny * (g.nz + MC3D_SAFE_CAP);
-            uint8_t classes[256];
-            const bool shared = index_classes(i, max_tissue[i], props, jobs, njobs, classes);
             e = pool_alloc(&p->d_cells[i], 2 * nmap, p->device, p->stream);
             if (e == cudaSuccess)
-                e = launch_safe_distance(p->d_grids[i], g.nx, g.ny, g.nz, map_t, tmp,
-                                         tmp + max_map, p->stream);
-            if (e == cudaSuccess && shared)
-                e = launch_index_classes(p->d_grids[i], (int64_t)g.nx * g.ny * g.nz, classes, cls,
-                                         p->stream);
-            if (e == cudaSuccess && shared)
-                e = launch_safe_distance(cls, g.nx, g.ny, g.nz, map_n, tmp, tmp + max_map,
-                                         p->stream);
-            if (e == cudaSuccess)
-                e = launch_pack_cells(p->d_grids[i], map_t, shared ? map_n : map_t, g.nx, g.ny,
-                                      g.nz, p->d_cells[i], p->stream);
+                e = launch_cells(p->d_grids[i], g.nx, g.ny, g.nz, c.one_tissue,
+                                 c.shared ? c.classes : nullptr, c.one_index, p->d_cells[i], tmp,
+                                 p->stream);
             gh[i].cells = p->d_cells[i];
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
-        cudaFreeAsync(tmp, p->stream);
+        if (tmp) cudaFreeAsync(tmp, p->stream);
         PLAN_TRY(e);
     }
     PLAN_TRY(pool_alloc(&p->d_geoms, sizeof(GeomDev) * ngeoms, p->device, p->stream));
@@ -885,12 +893,14 @@ int mc3d_safe_distance(const uint8_t *tissue, int32_t nx, int32_t ny, int32_t nz
     CUDA_TRY(cudaSetDevice(device));
     const size_t nv = (size_t)nx * ny * nz;
     const size_t nm = (size_t)nx * ny * (nz + MC3D_SAFE_CAP);
+    /* scratch | map | grid: the scratch is read in words */
+    const size_t scratch = safe_distance_scratch(nx, ny, nz, false);
     uint8_t *d = nullptr;
-    cudaError_t e = cudaMalloc(&d, nv + 3 * nm); /* grid | map | two scratch maps */
-    if (e == cudaSuccess) e = cudaMemcpy(d, tissue, nv, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = launch_safe_distance(d, nx, ny, nz, d + nv, d + nv + nm, d + nv + 2 * nm, nullptr);
-    if (e == cudaSuccess) e = cudaMemcpy(radius, d + nv, nm, cudaMemcpyDeviceToHost);
+    cudaError_t e = cudaMalloc(&d, scratch + nm + nv);
+    uint8_t *d_map = d + scratch, *d_grid = d_map + nm;
+    if (e == cudaSuccess) e = cudaMemcpy(d_grid, tissue, nv, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = launch_safe_distance(d_grid, nx, ny, nz, d_map, d, nullptr);
+    if (e == cudaSuccess) e = cudaMemcpy(radius, d_map, nm, cudaMemcpyDeviceToHost);
     cudaFree(d);
     if (e != cudaSuccess) return fail(MC3D_ERR_CUDA, "safe distance: %s", cudaGetErrorString(e));
     return MC3D_OK;

@@ -50,19 +50,20 @@ cudaError_t launch_seed_scan(const JobDev *jobs, int njobs, const uint32_t *mult
 /* states of streams [first, first+count) of job 0 of `jobs` */
 cudaError_t launch_seed_dump(const KernelParams &P, int64_t first, int64_t count,
                              uint64_t *x_out, uint32_t *a_out, cudaStream_t stream);
-/* safe-distance map of a tissue grid (merged steps): out, tmp_a and tmp_b hold
- * nx * ny * (nz + MC3D_SAFE_CAP) bytes each */
-cudaError_t launch_safe_distance(const uint8_t *tissue, int nx, int ny, int nz, uint8_t *out,
-                                 uint8_t *tmp_a, uint8_t *tmp_b, cudaStream_t stream);
-/* packed cells (tissue | box radius << 8) from the safe distances of the tissue grid
- * (radius) and of its refractive-index classes (radius_n; the same map when every
- * tissue has its own class) */
-cudaError_t launch_pack_cells(const uint8_t *tissue, const uint8_t *radius,
-                              const uint8_t *radius_n, int nx, int ny, int nz, uint16_t *cells,
-                              cudaStream_t stream);
-/* out[v] = classes[tissue[v]] for nv voxels (classes: 256 entries, host memory) */
-cudaError_t launch_index_classes(const uint8_t *tissue, int64_t nv, const uint8_t *classes,
-                                 uint8_t *out, cudaStream_t stream);
+/* bytes of scratch that the two launches below need for a grid: two maps of whole
+ * words a row, three with the distances of the refractive-index classes */
+size_t safe_distance_scratch(int nx, int ny, int nz, bool index_map);
+/* safe-distance map of a tissue grid: nx * ny * (nz + MC3D_SAFE_CAP) bytes */
+cudaError_t launch_safe_distance(const uint8_t *tissue, int nx, int ny, int nz, uint8_t *radius,
+                                 uint8_t *scratch, cudaStream_t stream);
+/* Packed cells (tissue | box radius << 8) of a grid, nz + MC3D_SAFE_CAP slices.
+ * one_tissue: the tissue of a grid that holds no other, else -1 (no scratch then).
+ * classes (256 entries, host memory): the refractive-index class of each tissue where
+ * some tissues share one, else NULL; one_index: every tissue of the grid is of one
+ * class, so that only the faces bound its index (no map of the classes then). */
+cudaError_t launch_cells(const uint8_t *tissue, int nx, int ny, int nz, int one_tissue,
+                         const uint8_t *classes, bool one_index, uint16_t *cells, uint8_t *scratch,
+                         cudaStream_t stream);
 cudaError_t launch_mwc_draws(const uint64_t *x, const uint32_t *a, int64_t ngen, int64_t n,
                              float *out, cudaStream_t stream);
 
