@@ -53,7 +53,7 @@ struct JobDev {
     int32_t beam;         /* 0 uniform over the top face, 1 pencil at the centre */
     int32_t rej_offset;   /* slice of the rejection list */
     int32_t rej_count;
-    int32_t pad;
+    int32_t index;        /* the caller's number of the job, whose totals it has */
 };
 
 /* A stream whose seeding attempt(s) were rejected (gpumcml_rng/gpumcml_rng.cu:100)
@@ -72,7 +72,7 @@ struct PhotonRecord {
 };
 
 struct KernelParams {
-    const JobDev *jobs;
+    const JobDev *jobs; /* in the order in which their streams are taken */
     const GeomDev *geoms;
     const float4 *props_table; /* 3 float4 per tissue (see photon_step), sets back to back */
     const uint32_t *multipliers; /* safe-prime table, entry 0 = seeding multiplier */
