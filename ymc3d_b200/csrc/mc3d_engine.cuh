@@ -139,6 +139,7 @@ struct FloatTable {
     }
     /* thresholds of src/mc3d_types.h:11-18, see the constants below */
     static __device__ __forceinline__ bool w_below_threshold(float w) { return w <= 0x1.a36e2ep-14f; }
+    static __device__ __forceinline__ bool w_above_threshold(float w) { return w > 0x1.a36e2ep-14f; }
     static __device__ __forceinline__ bool uz_within(float u) { return u <= 0x1.fffeb0p-1f; }
     static __device__ __forceinline__ float roulette_survivor(float w)
     {
@@ -584,10 +585,19 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
     nuy = (!hit) ? spin.uy : nuy;
     nuz = (!hit) ? spin.uz : nuz;
 
-    /* the normalisation and the next free path, again for the cell load's time: both are
-     * repeated below for the few steps that change them (a lone photon's step 3 % sooner) */
-    R norm = M::rsqrt(M::mad(nuz, nuz, M::mad(nuy, nuy, M::mul(nux, nux))));
-    R newS = -M::log((R)(1.0f - mc3d_u32_to_float_rz(e_s) * 0x1p-32f));
+    /* The normalised direction and the next free path.  Fast math computes them here,
+     * while the load is under way, and again for the few steps that change them (a lone
+     * photon's step takes 3 % less); where they are long, once, at the step's end. */
+    R ux, uy, uz, newS;
+    auto finish = [&]() {
+        const R norm = M::rsqrt(M::mad(nuz, nuz, M::mad(nuy, nuy, M::mul(nux, nux))));
+        ux = M::mul(nux, norm);
+        uy = M::mul(nuy, norm);
+        uz = M::mul(nuz, norm);
+        newS = -M::log((R)(1.0f - mc3d_u32_to_float_rz(e_s) * 0x1p-32f));
+    };
+    if (M::kFast) finish();
+
     /* What few steps need, behind one test: another tissue, a weight below the
      * roulette's threshold, air, components that snap to zero, the scattering of a
      * photon along the z axis, and the lateral faces.  The cell is looked up above
@@ -595,13 +605,16 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
     const R zero_thresh = M::zero_threshold();
     const bool steep = !M::uz_within(M::fabs(p.uz));
     const uint32_t changed = (uint32_t)(next_tissue ^ p.tissue) & 0xffu;
-    if (M::rare(changed, W, mu_t, p.uz, M::fmin(M::fabs(nux), M::fmin(M::fabs(nuy), M::fabs(nuz))),
-                newx, g.Lx, newy, g.Ly)) {
+    const R least_u = M::fmin(M::fabs(nux), M::fmin(M::fabs(nuy), M::fabs(nuz)));
+    if (M::rare(changed, W, mu_t, p.uz, least_u, newx, g.Lx, newy, g.Ly)) {
         bool refl = false;
-        bool again = steep && !hit;
-        const R ni = M::n(tt);
-        const R nt = M::n(tab + MC3D_TAB_STRIDE * (JUMP ? (next_tissue & 0xff) : next_tissue));
-        if (ni != nt) { /* Fresnel, src/mc3d_gpu.cu:226-257 */
+        bool again = steep && !hit;   /* the scattering anew */
+        bool redo = steep | (least_u < zero_thresh); /* the normalisation anew */
+        const bool lateral = !(newx > 0) | !(newx < g.Lx) | !(newy > 0) | !(newy < g.Ly);
+        if (((next_tissue ^ p.tissue) & 0xff) != 0 &&
+            M::n(tt) != M::n(tab + MC3D_TAB_STRIDE * (next_tissue & 0xff))) {
+            /* Fresnel, src/mc3d_gpu.cu:226-257 */
+            const R ni = M::n(tt), nt = M::n(tab + MC3D_TAB_STRIDE * (next_tissue & 0xff));
             const bool mx = p.i != nexti, my = p.j != nextj, mz = p.k != nextk;
             R cos_ai = mx ? p.ux : (my ? p.uy : p.uz);
             cos_ai = M::fabs(cos_ai);
@@ -662,59 +675,68 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
                 nuz = refl ? (mz ? -p.uz : p.uz) : tz;
             }
             again = !hit; /* an interaction that rounded onto the face */
+            redo = true;
             acc[T_FRESNEL] += 1;
         }
-        /* Russian roulette, src/mc3d_gpu.cu:275-277 */
-        if (M::w_below_threshold(W) && !hit && mu_t != 0) {
-            const float eps = mc3d_u32_to_float_rz(e_rr) * 0x1p-32f;
-            const R newW = (eps < MC3D_SURVIVAL_LT_F) ? M::roulette_survivor(W) : (R)0;
-            /* absorbed weight is booked at the photon's end as Q(W0) - Q(W_end) - lost;
-             * a roulette event moves its share from there to the roulette tallies */
-            if (newW == 0) {
-                uint64_t k = M::qw(W);
-                acc[T_RR_KILLED] += k;
-                acc[T_ABSORBED] -= k;
-            } else {
-                uint64_t c = M::qw(newW) - M::qw(W);
-                acc[T_RR_CREATED] += c;
-                acc[T_ABSORBED] += c;
+        if (!M::w_above_threshold(W) | (mu_t == 0)) {
+            /* Russian roulette, src/mc3d_gpu.cu:275-277 */
+            if (M::w_below_threshold(W) && !hit && mu_t != 0) {
+                const float eps = mc3d_u32_to_float_rz(e_rr) * 0x1p-32f;
+                const R newW = (eps < MC3D_SURVIVAL_LT_F) ? M::roulette_survivor(W) : (R)0;
+                /* absorbed weight is booked at the photon's end as Q(W0) - Q(W_end) - lost;
+                 * a roulette event moves its share from there to the roulette tallies */
+                if (newW == 0) {
+                    uint64_t k = M::qw(W);
+                    acc[T_RR_KILLED] += k;
+                    acc[T_ABSORBED] -= k;
+                } else {
+                    uint64_t c = M::qw(newW) - M::qw(W);
+                    acc[T_RR_CREATED] += c;
+                    acc[T_ABSORBED] += c;
+                }
+                W = newW;
             }
-            W = newW;
+            if (W <= 0 || mu_t == 0) { /* freeze (:303-311): the photon stays where it is */
+                p.W = W;
+                p.s = hit ? s : p.s - p.s;
+                *lat_mirror = false;
+                if (!refl && !(p.x > 0 && p.x < g.Lx && p.y > 0 && p.y < g.Ly))
+                    *lat_mirror = mirror<M>(&p.x, &p.ux, g.Lx) || mirror<M>(&p.y, &p.uy, g.Ly);
+                return true;
+            }
+            if (!(W > 0)) { /* NaN weight: no free path, -log(1) */
+                e_s = 0;
+                redo = true;
+            }
         }
-        if (W <= 0 || mu_t == 0) { /* freeze (:303-311): the photon stays where it is */
-            p.W = W;
-            p.s = hit ? s : p.s - p.s;
-            *lat_mirror = false;
-            if (!refl && !(p.x > 0 && p.x < g.Lx && p.y > 0 && p.y < g.Ly))
-                *lat_mirror = mirror<M>(&p.x, &p.ux, g.Lx) || mirror<M>(&p.y, &p.uy, g.Ly);
-            return true;
+        if (redo) {
+            if (again) {
+                const Spin<R> sp = scatter<M, SPLIT_SIN2>(tt, p, e_hg, e_phi);
+                nux = steep ? M::mul(sp.sintheta, sp.cosphi) : sp.ux;
+                nuy = steep ? M::mul(sp.sintheta, sp.sinphi) : sp.uy;
+                nuz = steep ? M::copysign(sp.costheta, M::mul(sp.costheta, p.uz)) : sp.uz;
+            }
+            nux = (M::fabs(nux) < zero_thresh) ? 0 : nux;
+            nuy = (M::fabs(nuy) < zero_thresh) ? 0 : nuy;
+            nuz = (M::fabs(nuz) < zero_thresh) ? 0 : nuz;
+            if (M::kFast) finish();
         }
-        if (!(W > 0)) e_s = 0; /* NaN weight: no free path, -log(1) */
-        if (again) {
-            const Spin<R> sp = scatter<M, SPLIT_SIN2>(tt, p, e_hg, e_phi);
-            nux = steep ? M::mul(sp.sintheta, sp.cosphi) : sp.ux;
-            nuy = steep ? M::mul(sp.sintheta, sp.sinphi) : sp.uy;
-            nuz = steep ? M::copysign(sp.costheta, M::mul(sp.costheta, p.uz)) : sp.uz;
-        }
-        nux = (M::fabs(nux) < zero_thresh) ? 0 : nux;
-        nuy = (M::fabs(nuy) < zero_thresh) ? 0 : nuy;
-        nuz = (M::fabs(nuz) < zero_thresh) ? 0 : nuz;
-        /* mirrors, short-circuited as in src/mc3d_gpu.cu:330.  A mirror turns its
-         * component before the normalisation, which keeps the sign. */
-        refl = refl || mirror<M>(&newx, &nux, g.Lx) || mirror<M>(&newy, &nuy, g.Ly);
+        /* mirrors, short-circuited as in src/mc3d_gpu.cu:330; a mirror turns its component
+         * before or after the normalisation, which keeps the sign */
+        if (lateral)
+            refl = refl || mirror<M>(&newx, M::kFast ? &ux : &nux, g.Lx) ||
+                   mirror<M>(&newy, M::kFast ? &uy : &nuy, g.Ly);
         if (hit && refl) { /* a reflected photon keeps its voxel (:334-339) */
             nexti = p.i;
             nextj = p.j;
             nextk = p.k;
             next_tissue = p.tissue;
         }
-        norm = M::rsqrt(M::mad(nuz, nuz, M::mad(nuy, nuy, M::mul(nux, nux))));
-        newS = -M::log((R)(1.0f - mc3d_u32_to_float_rz(e_s) * 0x1p-32f));
     }
-    p.ux = M::mul(nux, norm);
-    p.uy = M::mul(nuy, norm);
-    p.uz = M::mul(nuz, norm);
-
+    if (!M::kFast) finish();
+    p.ux = ux;
+    p.uy = uy;
+    p.uz = uz;
     p.s = hit ? s : newS;
     p.W = W;
     p.x = newx;
@@ -920,17 +942,8 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
     bool drained = false; /* no stream left to take */
     int psteps = 0; /* steps of the photon before its present chunk */
     unsigned long long *amap = nullptr;
-    bool drain = false; /* the block is past the last stream */
-    int turn = 0;
-
-    /* One iteration is one 45-step chunk, the reference's launch.  A photon starts
-     * only at a chunk's start, as a reference slot starts only at a launch boundary:
-     * a lane whose photon ended waits out the rest of the chunk (the reference's
-     * masked steps).  The two warp barriers make that wait real: without them a lane
-     * that leaves the step loop early runs on alone, and from then on the warp steps
-     * in pieces (22.5 lanes a step and 4.7 a chunk's end instead of 30 and 30, layered
-     * 1e6 photons).  Lanes without a photon stay in the loop until the warp has none. */
-    for (;;) {
+    /* a lane without photons left in its stream takes the next stream */
+    auto take_stream = [&]() {
         if (!alive && !drained) {
             while (left == 0) {
                 drained = P.cancel && *((volatile const int *)P.cancel);
@@ -953,7 +966,10 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
                 rx = stream_seed(P, jb, local, ra);
             }
         }
-        if (!alive && !drained) {
+    };
+    /* a lane without a photon starts the next of its stream */
+    auto start_photon = [&]() {
+        if (!alive && left != 0) {
             const GeomDev &g = ONE_GEOM ? P.geom0 : *gp;
             /* photontrack_reinitialize, src/mc3d_gpu.cu:74-111 */
             if (P.jobs[job].beam == 0) {
@@ -975,67 +991,14 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
             alive = true;
             left--;
         }
-        /* The drain.  Once the streams run out, lanes fall idle one by one and the last
-         * photons of a launch, up to 15 times the mean length, would leave warps stepping
-         * for one or two lanes each and, by sharing an SM, slowing one another.  So from
-         * then on the block's warps meet at each chunk's start and, whenever its photons
-         * fit into fewer warps, close ranks: at most seven times, a photon's state passing
-         * through shared memory.  Where a photon is stepped changes nothing in its
-         * trajectory. */
-        if (!drain) {
-            if (drained) sh_drain = 1;
-            drain = __any_sync(0xffffffffu, sh_drain != 0);
-        }
-        if (drain) {
-            const unsigned live = __ballot_sync(0xffffffffu, alive);
-            int *count = sh_live[turn];
-            turn ^= 1; /* the other half is written only after all have read this one */
-            if ((threadIdx.x & 31) == 0) count[threadIdx.x >> 5] = __popc(live);
-            __syncthreads();
-            int total = 0, before = 0, warps = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-                if (w == (int)(threadIdx.x >> 5)) before = total;
-                total += count[w];
-                warps += count[w] != 0;
-            }
-            if (total == 0) break;
-            if ((total + 31) / 32 < warps) {
-                /* the rows become free of tallies, then carry the photons */
-                if (job >= 0) acc_flush(acc, job_totals(P, job));
-                const int64_t my_left = left, my_local = local;
-                __syncthreads();
-                if (alive) {
-                    const int to = before + __popc(live & ((1u << (threadIdx.x & 31)) - 1u));
-                    const Acc other{sh_rows + MC3D_THREAD_WORDS * to};
-                    *reinterpret_cast<ParkedT<R> *>(other.row) = ParkedT<R>{
-                        rx, p.x, p.y, p.z, p.ux, p.uy, p.uz, p.W, p.s, p.i, p.j, p.k,
-                        p.tissue, ra, psteps, job};
-                    other.left() = my_left;
-                    other.local() = my_local;
-                }
-                __syncthreads();
-                alive = (int)threadIdx.x < total;
-                drained = !alive;
-                if (alive) {
-                    const ParkedT<R> q = *reinterpret_cast<const ParkedT<R> *>(acc.row);
-                    rx = q.rx;
-                    p.x = q.x; p.y = q.y; p.z = q.z;
-                    p.ux = q.ux; p.uy = q.uy; p.uz = q.uz;
-                    p.W = q.W; p.s = q.s;
-                    p.i = q.i; p.j = q.j; p.k = q.k;
-                    p.tissue = q.tissue;
-                    ra = q.ra;
-                    psteps = q.psteps;
-                    job = q.job;
-                    gp = sh_geom + P.jobs[job].geom;
-                    tab = sh_tab + P.jobs[job].props_offset;
-                    if (AMAP) amap = P.amap + P.jobs[job].amap_offset;
-                }
-                asm volatile("" ::: "memory"); /* the row is read before it is cleared */
-                acc_clear(acc);
-            }
-        }
-
+    };
+    /* One chunk of 45 steps, the reference's launch, and its end.  A photon starts only at
+     * a chunk's start, as a reference slot starts only at a launch boundary: a lane whose
+     * photon ended waits out the rest of the chunk (the reference's masked steps).  The
+     * barrier after the steps makes that wait real: without it a lane that leaves the step
+     * loop early runs on alone, and from then on the warp steps in pieces (4.7 lanes a
+     * chunk's end instead of 32, layered 1e6 photons). */
+    auto run_chunk = [&]() {
         const GeomDev &g = ONE_GEOM ? P.geom0 : *gp;
         /* The chunk's steps, fewer where the step cap comes first.  Merged steps: the
          * quickfix must see the boundary distance of the reference's one-voxel DDA
@@ -1061,7 +1024,7 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
             stop = cap;
         }
         __syncwarp();
-        if (!alive) continue;
+        if (!alive) return;
         psteps += chunk;
 
         bool done = false;
@@ -1146,6 +1109,94 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
                 P.photon_log[pid] = r;
             }
             alive = false;
+        }
+    };
+
+    /* The drain.  Once the streams run out, lanes fall idle one by one and the last
+     * photons of a launch, up to 15 times the mean length, would leave warps stepping
+     * for one or two lanes each and, by sharing an SM, slowing one another.  So from
+     * then on the block's warps meet at each chunk's start and, whenever its photons
+     * fit into fewer warps, close ranks: at most seven times, a photon's state passing
+     * through shared memory.  Where a photon is stepped changes nothing in its
+     * trajectory. */
+    int turn = 0;
+    auto close_ranks = [&]() { /* false when the block has no photon left */
+        const unsigned live = __ballot_sync(0xffffffffu, alive);
+        int *count = sh_live[turn];
+        turn ^= 1; /* the other half is written only after all have read this one */
+        if ((threadIdx.x & 31) == 0) count[threadIdx.x >> 5] = __popc(live);
+        __syncthreads();
+        int total = 0, before = 0, warps = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
+            if (w == (int)(threadIdx.x >> 5)) before = total;
+            total += count[w];
+            warps += count[w] != 0;
+        }
+        if (total == 0) return false;
+        if ((total + 31) / 32 < warps) {
+            /* the rows become free of tallies, then carry the photons */
+            if (job >= 0) acc_flush(acc, job_totals(P, job));
+            const int64_t my_left = left, my_local = local;
+            __syncthreads();
+            if (alive) {
+                const int to = before + __popc(live & ((1u << (threadIdx.x & 31)) - 1u));
+                const Acc other{sh_rows + MC3D_THREAD_WORDS * to};
+                *reinterpret_cast<ParkedT<R> *>(other.row) = ParkedT<R>{
+                    rx, p.x, p.y, p.z, p.ux, p.uy, p.uz, p.W, p.s, p.i, p.j, p.k,
+                    p.tissue, ra, psteps, job};
+                other.left() = my_left;
+                other.local() = my_local;
+            }
+            __syncthreads();
+            alive = (int)threadIdx.x < total;
+            if (alive) {
+                const ParkedT<R> q = *reinterpret_cast<const ParkedT<R> *>(acc.row);
+                rx = q.rx;
+                p.x = q.x; p.y = q.y; p.z = q.z;
+                p.ux = q.ux; p.uy = q.uy; p.uz = q.uz;
+                p.W = q.W; p.s = q.s;
+                p.i = q.i; p.j = q.j; p.k = q.k;
+                p.tissue = q.tissue;
+                ra = q.ra;
+                psteps = q.psteps;
+                job = q.job;
+                gp = sh_geom + P.jobs[job].geom;
+                tab = sh_tab + P.jobs[job].props_offset;
+                if (AMAP) amap = P.amap + P.jobs[job].amap_offset;
+            } else {
+                left = 0;
+            }
+            asm volatile("" ::: "memory"); /* the row is read before it is cleared */
+            acc_clear(acc);
+        }
+        return true;
+    };
+
+    if (M::kFast) {
+        /* two loops: with the drain's code in it the compiler reloads the launch's
+         * constants in every step (6.6 of 196 instructions) */
+        for (;;) {
+            take_stream();
+            start_photon();
+            if (drained) sh_drain = 1;
+            if (__any_sync(0xffffffffu, sh_drain != 0)) break;
+            run_chunk();
+        }
+        for (;;) {
+            start_photon();
+            if (!close_ranks()) break;
+            run_chunk();
+        }
+    } else {
+        /* one loop: the steps, several times as long, want the registers (FP64, 2e5
+         * photons: 48.8 ms, with two loops 50.1) */
+        for (bool drain = false;;) {
+            if (!drain) take_stream();
+            start_photon();
+            if (drained) sh_drain = 1;
+            drain = drain || __any_sync(0xffffffffu, sh_drain != 0);
+            if (drain && !close_ranks()) break;
+            run_chunk();
         }
     }
     if (job >= 0) acc_flush(acc, job_totals(P, job));
