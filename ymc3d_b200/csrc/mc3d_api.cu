@@ -106,6 +106,7 @@ cudaError_t pool_alloc(T **ptr, size_t bytes, int device, cudaStream_t s)
  * 227 KB per block, less 34 KB of rows for 256 threads) */
 const int kMaxSharedTable = 192 * 1024;
 const int64_t kMaxAttempts = 4096;       /* seeding attempts per stream before giving up */
+const int64_t kMaxKeptSeeds = 1ll << 27; /* streams whose states a plan keeps (1 GiB) */
 
 /* seeding-generator constants for multiplier `begin` (see mc3d_rng.h) */
 void make_seed_consts(uint32_t begin, mc3d_seed_consts *c)
@@ -306,6 +307,7 @@ struct mc3d_plan {
     float4 *d_props = nullptr;
     uint32_t *d_mult = nullptr;
     RejectionDev *d_rej = nullptr;
+    uint64_t *d_seeds = nullptr;
     unsigned long long *d_tally = nullptr; /* drs | drs_sq | trans | totals | counter */
     unsigned long long *d_amap = nullptr;  /* absorption map, all jobs' voxels */
     std::vector<int64_t> job_voxels;
@@ -334,7 +336,7 @@ static void plan_free(mc3d_plan *p)
         std::vector<void *> bufs(p->d_grids.begin(), p->d_grids.end());
         bufs.insert(bufs.end(), p->d_cells.begin(), p->d_cells.end());
         for (void *b : {(void *)p->d_jobs, (void *)p->d_geoms, (void *)p->d_props,
-                        (void *)p->d_mult, (void *)p->d_rej, (void *)p->d_tally,
+                        (void *)p->d_mult, (void *)p->d_rej, (void *)p->d_seeds, (void *)p->d_tally,
                         (void *)p->d_amap, (void *)p->d_log})
             bufs.push_back(b);
         for (void *b : bufs)
@@ -635,8 +637,13 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
                         p->stream));
     unsigned long long *first_reject = p->d_tally; /* scratch reuse before the first run */
     PLAN_TRY(cudaMemsetAsync(first_reject, 0xff, sizeof(unsigned long long) * njobs, p->stream));
+    /* the streams' states, unless they would take more than 1 GiB or the memory is not
+     * there: then each stream computes its own when it starts */
+    if (stream_base > 0 && stream_base <= kMaxKeptSeeds &&
+        pool_alloc(&p->d_seeds, sizeof(uint64_t) * stream_base, p->device, p->stream) != cudaSuccess)
+        cudaGetLastError();
     PLAN_TRY(launch_seed_scan(p->d_jobs, njobs, p->d_mult, table_len, sc, scan_base,
-                              first_reject, p->stream));
+                              first_reject, p->d_seeds, p->stream));
     std::vector<unsigned long long> fr(njobs);
     PLAN_TRY(cudaMemcpyAsync(fr.data(), first_reject, sizeof(unsigned long long) * njobs,
                              cudaMemcpyDeviceToHost, p->stream));
@@ -737,6 +744,7 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
     P.props_table = p->d_props;
     P.multipliers = p->d_mult;
     P.rejections = p->d_rej;
+    P.seeds = any_rej ? nullptr : p->d_seeds;
     P.drs = p->d_tally;
     P.drs_sq = p->d_tally + p->total_bins;
     P.trans = p->d_tally + 2 * p->total_bins;

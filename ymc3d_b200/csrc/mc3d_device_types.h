@@ -77,6 +77,7 @@ struct KernelParams {
     const float4 *props_table; /* 3 float4 per tissue (see photon_step), sets back to back */
     const uint32_t *multipliers; /* safe-prime table, entry 0 = seeding multiplier */
     const RejectionDev *rejections;
+    const uint64_t *seeds;      /* initial state of every stream launched, or NULL */
     unsigned long long *drs;    /* sum Q(W) of reflected photons per surface bin */
     unsigned long long *drs_sq; /* sum Q(W^2) */
     unsigned long long *trans;  /* sum Q(W) of photons frozen below the surface */

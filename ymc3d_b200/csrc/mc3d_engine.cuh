@@ -963,7 +963,7 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
                 local = gs - jb.stream_base + jb.stream_first;
                 left = jb.per_stream + (local < jb.remainder ? 1 : 0);
                 ra = stream_multiplier(P, local);
-                rx = stream_seed(P, jb, local, ra);
+                rx = P.seeds ? P.seeds[gs] : stream_seed(P, jb, local, ra);
             }
         }
     };

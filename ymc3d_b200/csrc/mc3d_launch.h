@@ -43,10 +43,12 @@ cudaError_t smem_limit_photon_exact(size_t smem);
 cudaError_t attributes_photon_fast(cudaFuncAttributes *attr);
 cudaError_t attributes_photon_exact(cudaFuncAttributes *attr);
 
-/* first rejected seeding attempt per job, assuming none before it (UINT64_MAX if none) */
+/* first rejected seeding attempt per job, assuming none before it (UINT64_MAX if none);
+ * seeds, if not NULL, gets the state of every launched stream under the same assumption */
 cudaError_t launch_seed_scan(const JobDev *jobs, int njobs, const uint32_t *mult,
                              int64_t nmult, const mc3d_seed_consts &sc, int64_t total_streams,
-                             unsigned long long *first_reject, cudaStream_t stream);
+                             unsigned long long *first_reject, uint64_t *seeds,
+                             cudaStream_t stream);
 /* states of streams [first, first+count) of job 0 of `jobs` */
 cudaError_t launch_seed_dump(const KernelParams &P, int64_t first, int64_t count,
                              uint64_t *x_out, uint32_t *a_out, cudaStream_t stream);

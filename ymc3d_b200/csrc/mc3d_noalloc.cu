@@ -228,7 +228,7 @@ extern "C" int mc3d_run_noalloc(const mc3d_geom *geom, const mc3d_props *props,
     mc3d_seed_consts sc;
     make_seed_consts_host(table[0], &sc);
     NA_TRY(launch_seed_scan((const JobDev *)(base + kOffJob), 1, (const uint32_t *)(base + kOffMult),
-                            table_len, sc, first + count, words + 1, s));
+                            table_len, sc, first + count, words + 1, nullptr, s));
     unsigned long long hw[3];
     NA_TRY(cudaMemcpyAsync(hw, words, sizeof hw, cudaMemcpyDeviceToHost, s));
     NA_TRY(cudaStreamSynchronize(s));

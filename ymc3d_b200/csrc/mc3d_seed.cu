@@ -7,6 +7,8 @@
  * per-stream state in memory.  The only sequential coupling is a rejected attempt,
  * which shifts every later stream by one attempt; the scan below finds the first
  * rejected stream of each job and the host lists the (rare) rejections from there.
+ * Without a rejection the states it computes are the streams' own, and a plan keeps
+ * them (8 bytes each) for its launches: about 500 instructions less per photon.
  */
 #include <climits>
 #include "mc3d_engine.cuh"
@@ -16,7 +18,8 @@ namespace mc3d {
 
 __global__ void seed_scan_kernel(const JobDev *jobs, int njobs, const uint32_t *mult,
                                  int64_t nmult, const __grid_constant__ mc3d_seed_consts sc,
-                                 int64_t total_streams, unsigned long long *first_reject)
+                                 int64_t total_streams, unsigned long long *first_reject,
+                                 uint64_t *seeds)
 {
     for (int64_t gs = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; gs < total_streams;
          gs += (int64_t)gridDim.x * blockDim.x) {
@@ -32,19 +35,22 @@ __global__ void seed_scan_kernel(const JobDev *jobs, int njobs, const uint32_t *
         uint64_t xs = mc3d_seed_jump(&sc, jobs[j].seed, (uint64_t)local);
         uint64_t st = mc3d_seed_attempt(xs, sc.begin, fora);
         if (!mc3d_seed_valid(st, fora)) atomicMin(first_reject + j, (unsigned long long)local);
+        if (seeds && local >= jobs[j].stream_first)
+            seeds[jobs[j].stream_base + local - jobs[j].stream_first] = st;
     }
 }
 
 cudaError_t launch_seed_scan(const JobDev *jobs, int njobs, const uint32_t *mult, int64_t nmult,
                              const mc3d_seed_consts &sc, int64_t total_streams,
-                             unsigned long long *first_reject, cudaStream_t stream)
+                             unsigned long long *first_reject, uint64_t *seeds,
+                             cudaStream_t stream)
 {
     if (total_streams <= 0) return cudaSuccess;
     int block = 256;
     int64_t want = (total_streams + block - 1) / block;
     int grid = (int)(want < 148 * 64 ? want : 148 * 64);
     seed_scan_kernel<<<grid, block, 0, stream>>>(jobs, njobs, mult, nmult, sc, total_streams,
-                                                 first_reject);
+                                                 first_reject, seeds);
     return cudaGetLastError();
 }
 
