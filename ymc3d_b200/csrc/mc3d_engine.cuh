@@ -721,11 +721,23 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
             nuz = (M::fabs(nuz) < zero_thresh) ? 0 : nuz;
             if (M::kFast) finish();
         }
-        /* mirrors, short-circuited as in src/mc3d_gpu.cu:330; a mirror turns its component
-         * before or after the normalisation, which keeps the sign */
-        if (lateral)
-            refl = refl || mirror<M>(&newx, M::kFast ? &ux : &nux, g.Lx) ||
-                   mirror<M>(&newy, M::kFast ? &uy : &nuy, g.Ly);
+        /* The mirrors, short-circuited as in src/mc3d_gpu.cu:330, both axes at once.  A
+         * mirror turns its component before or after the normalisation, which keeps the
+         * sign. */
+        if (lateral && !refl) {
+            R &mx = M::kFast ? ux : nux, &my = M::kFast ? uy : nuy;
+            const bool in_x = (newx >= g.Lx) | (newx <= 0);
+            const bool in_y = !in_x & ((newy >= g.Ly) | (newy <= 0));
+            const R length = in_x ? (R)g.Lx : (R)g.Ly;
+            R c = in_x ? newx : newy;
+            c = c >= length ? 2 * length - c : c;
+            c = M::fabs(c);
+            newx = in_x ? c : newx;
+            newy = in_y ? c : newy;
+            mx = in_x ? -mx : mx;
+            my = in_y ? -my : my;
+            refl = in_x | in_y;
+        }
         if (hit && refl) { /* a reflected photon keeps its voxel (:334-339) */
             nexti = p.i;
             nextj = p.j;
