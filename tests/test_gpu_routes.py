@@ -16,7 +16,7 @@ import numpy as np
 import pytest
 
 import ymc3d_b200 as m
-from helpers import residual, safe_distance_bruteforce
+from helpers import oracle_job, residual, safe_distance_bruteforce
 from ymc3d_b200 import workloads
 
 pytestmark = pytest.mark.gpu
@@ -153,3 +153,21 @@ def test_fast_tallies_are_the_recorded_ones(table, name):
     geoms, props, jobs, how = fast_cases()[name]
     want = json.loads(GOLDEN.read_text())[name]
     assert tallies(m.run(geoms, props, jobs, table=table, **how)) == want
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -58, 2.0 ** -66, 2.0 ** 64])
+@pytest.mark.parametrize("absorption", [False, True])
+def test_exact_divisions_at_the_range_ends(table, scale, absorption):
+    """Exact math divides by voxel sizes and mu_t through their reciprocals within
+    [2^-60, 2^60] and by IEEE division beyond: photon by photon the CPU transcription's
+    states on both sides (a layered medium scaled in length, and so in 1/mm)."""
+    g = workloads.layered_vessel_geometry(31, 28, 17, 0.11)
+    g = m.Geometry(g.tissue, 0.11 * scale, 0.13 * scale, 0.07 * scale)
+    p = m.OpticalProps.from_tissues([(a / scale, s / scale, gg, n)
+                                     for a, s, gg, n in workloads.LAYER_ROWS])
+    job = m.Job(0, 0, 600, 271828, "uniform")
+    r = m.run([g], [p], [job], table=table, math="exact", photon_log=True, max_steps=20_000,
+              absorption_map=absorption)[0]
+    o = oracle_job(g, p, job, table, photon_log=True, max_steps=20_000)
+    assert np.array_equal(_log(r), o["photon_log"].view(np.uint8).reshape(600, -1))
+    assert r.totals == o["totals"] and np.array_equal(r.drs, o["drs"])

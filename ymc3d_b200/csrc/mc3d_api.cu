@@ -305,6 +305,8 @@ struct mc3d_plan {
     JobDev *d_jobs = nullptr;
     GeomDev *d_geoms = nullptr;
     float4 *d_props = nullptr;
+    GeomDev64 *d_geoms64 = nullptr; /* FP64 stepping only */
+    double *d_props64 = nullptr;
     uint32_t *d_mult = nullptr;
     RejectionDev *d_rej = nullptr;
     uint64_t *d_seeds = nullptr;
@@ -336,7 +338,7 @@ static void plan_free(mc3d_plan *p)
         std::vector<void *> bufs(p->d_grids.begin(), p->d_grids.end());
         bufs.insert(bufs.end(), p->d_cells.begin(), p->d_cells.end());
         for (void *b : {(void *)p->d_jobs, (void *)p->d_geoms, (void *)p->d_props,
-                        (void *)p->d_mult, (void *)p->d_rej, (void *)p->d_seeds, (void *)p->d_tally,
+                        (void *)p->d_geoms64, (void *)p->d_props64, (void *)p->d_mult, (void *)p->d_rej, (void *)p->d_seeds, (void *)p->d_tally,
                         (void *)p->d_amap, (void *)p->d_log})
             bufs.push_back(b);
         for (void *b : bufs)
@@ -619,6 +621,28 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
     PLAN_TRY(pool_alloc(&p->d_props, sizeof(float4) * entries, p->device, p->stream));
     PLAN_TRY(cudaMemcpyAsync(p->d_props, tab.data(), sizeof(float4) * entries,
                              cudaMemcpyHostToDevice, p->stream));
+    std::vector<GeomDev64> gh64;
+    std::vector<double> tab64;
+    if (p->math == MC3D_MATH_F64) {
+        /* what the step would derive in double from the floats, computed once */
+        for (const GeomDev &g : gh)
+            gh64.push_back({g.dx, g.dy, g.dz, g.Lx, g.Ly, 1.0 / g.dx, 1.0 / g.dy, 1.0 / g.dz, g.nx,
+                            g.ny, g.nz, g.last_z, g.last_x, g.last_y, g.tissue, g.cells});
+        for (int i = 0; i < nprops; i++)
+            for (int t = 0; t < props[i].num_tissue_types; t++) {
+                const double mua = props[i].mua[t], mut = mua + (double)props[i].mus[t];
+                const double g = props[i].g[t];
+                for (double v : {mut, 1.0 / mut, mut > 0 ? mua / mut : 0.0, (double)props[i].n[t],
+                                 1 - g * g, 1 - g, 2 * g, 1 + g * g, 1.0 / (2 * g)})
+                    tab64.push_back(v);
+            }
+        PLAN_TRY(pool_alloc(&p->d_geoms64, sizeof(GeomDev64) * ngeoms, p->device, p->stream));
+        PLAN_TRY(cudaMemcpyAsync(p->d_geoms64, gh64.data(), sizeof(GeomDev64) * ngeoms,
+                                 cudaMemcpyHostToDevice, p->stream));
+        PLAN_TRY(pool_alloc(&p->d_props64, sizeof(double) * tab64.size(), p->device, p->stream));
+        PLAN_TRY(cudaMemcpyAsync(p->d_props64, tab64.data(), sizeof(double) * tab64.size(),
+                                 cudaMemcpyHostToDevice, p->stream));
+    }
     /* the lines that the jobs' streams use: stream i has line 1 + i mod (table_len - 1) */
     int64_t lines = 1;
     for (const JobDev &d : jh)
@@ -712,6 +736,20 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
                                               : smem_limit_photon_f64(max_dyn));
     }
     p->variant = (p->jump ? 0 : MC3D_VARIANT_VOXEL_STEPS) | (ngeoms == 1 ? MC3D_VARIANT_ONE_GEOM : 0);
+    if (p->math == MC3D_MATH_EXACT) {
+        /* division by reciprocal: a step's quotients and their residuals stay normal when
+         * the divisors are within [2^-60, 2^60]; a tissue without mu_t is never divided by */
+        bool wide = false;
+        auto check = [&](float d) { wide |= !(d >= 0x1p-60f && d <= 0x1p60f); };
+        for (const GeomDev &g : gh) {
+            check(g.dx);
+            check(g.dy);
+            check(g.dz);
+        }
+        for (int i = 0; i < entries; i += 3)
+            if (tab[i + 1].x != 0) check(tab[i + 1].x);
+        if (wide) p->variant |= MC3D_VARIANT_DIVIDE;
+    }
     /* 128 threads, of whose registers an SM holds 20 warps of the fast kernel (16 in
      * blocks of 256), unless the optical tables, of which each block has a copy, leave
      * room for more threads in larger blocks */
@@ -721,7 +759,7 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
         int n = 0;
         const size_t smem = photon_smem(entries, ngeoms, block);
         PLAN_TRY(p->math == MC3D_MATH_FAST ? occupancy_photon_fast(block, smem, &n, p->variant)
-                 : p->math == MC3D_MATH_EXACT ? occupancy_photon_exact(block, smem, &n)
+                 : p->math == MC3D_MATH_EXACT ? occupancy_photon_exact(block, smem, &n, p->variant)
                                               : occupancy_photon_f64(block, smem, &n, p->variant));
         if (n * block > bps * p->block || p->block == 0) {
             p->block = block;
@@ -742,6 +780,8 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
     P.geoms = p->d_geoms;
     P.geom0 = gh[0];
     P.props_table = p->d_props;
+    P.geoms64 = p->d_geoms64;
+    P.props64 = p->d_props64;
     P.multipliers = p->d_mult;
     P.rejections = p->d_rej;
     P.seeds = any_rej ? nullptr : p->d_seeds;
@@ -777,7 +817,7 @@ static int plan_enqueue(mc3d_plan *p, cudaStream_t s)
     if (p->math == MC3D_MATH_FAST)
         CUDA_TRY(launch_photon_fast(p->P, p->grid, p->block, p->smem, s, p->variant));
     else if (p->math == MC3D_MATH_EXACT)
-        CUDA_TRY(launch_photon_exact(p->P, p->grid, p->block, p->smem, s));
+        CUDA_TRY(launch_photon_exact(p->P, p->grid, p->block, p->smem, s, p->variant));
     else CUDA_TRY(launch_photon_f64(p->P, p->grid, p->block, p->smem, s, p->variant));
     return MC3D_OK;
 }

@@ -35,6 +35,15 @@ struct GeomDev {
     const uint16_t *cells; /* tissue | box radius << 8, nz + MC3D_SAFE_CAP slices (merged) */
 };
 
+/* The same for FP64 stepping: the float sizes and lengths as doubles, and the correctly
+ * rounded reciprocals of the sizes. */
+struct GeomDev64 {
+    double dx, dy, dz, Lx, Ly, rdx, rdy, rdz;
+    int nx, ny, nz, last_z, last_x, last_y;
+    const uint8_t *tissue;
+    const uint16_t *cells;
+};
+
 struct JobDev {
     int64_t stream_base; /* first global stream index of the job's launched range */
     int64_t stream_first; /* job-local index of that first stream (shards) */
@@ -75,6 +84,8 @@ struct KernelParams {
     const JobDev *jobs; /* in the order in which their streams are taken */
     const GeomDev *geoms;
     const float4 *props_table; /* 3 float4 per tissue (see photon_step), sets back to back */
+    const GeomDev64 *geoms64; /* FP64 stepping: descriptors and, per tissue, nine doubles */
+    const double *props64;    /* (mu_t, 1/mu_t, mua/mu_t, n, 1-g^2, 1-g, 2g, 1+g^2, 1/(2g)) */
     const uint32_t *multipliers; /* safe-prime table, entry 0 = seeding multiplier */
     const RejectionDev *rejections;
     const uint64_t *seeds;      /* initial state of every stream launched, or NULL */

@@ -35,6 +35,9 @@
 
 namespace mc3d {
 
+#define MC3D_TAB_STRIDE 3   /* float4 per tissue in the optical table */
+#define MC3D_TAB64_STRIDE 9 /* doubles per tissue in the FP64 one */
+
 /* ---------------------------------------------------------------- math policies
  * A policy fixes the transport arithmetic type (real) and how the elementary
  * operations are evaluated, and reads the per-tissue coefficients of the optical
@@ -124,6 +127,18 @@ struct PackedOps {
  * per step, precomputed on the host. */
 struct FloatTable {
     using real = float;
+    using Geom = GeomDev;
+    using Row = const float4 *; /* of the table in shared memory, MC3D_TAB_STRIDE a tissue */
+    static constexpr bool kShared = true; /* table and geometries are read from shared memory */
+    static __device__ __forceinline__ Row row(Row tab, int tissue) { return tab + MC3D_TAB_STRIDE * tissue; }
+    static __device__ __forceinline__ Row table(const KernelParams &, Row shared, int offset)
+    {
+        return shared + offset;
+    }
+    static __device__ __forceinline__ const Geom *geom(const KernelParams &, const GeomDev *shared, int i)
+    {
+        return shared + i;
+    }
     static __device__ __forceinline__ float n(const float4 *tt) { return tt[0].w; }
     static __device__ __forceinline__ float mu_t(const float4 *tt) { return tt[1].x; }
     /* mua / mu_t, 0 where mu_t is not positive */
@@ -180,13 +195,18 @@ struct MathExact : FloatTable {
     static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
     static __device__ __forceinline__ float mad(float a, float b, float c) { return a * b + c; }
     static __device__ __forceinline__ float div(float a, float b) { return a / b; }
-    /* a / b where the caller also holds r = 1/b: the exact policy divides */
-    static __device__ __forceinline__ float div_r(float a, float b, float) { return a / b; }
+    /* a / b, correctly rounded, by r = 1 / b correctly rounded, as MathF64::div_r */
+    static __device__ __forceinline__ float div_r(float a, float b, float r)
+    {
+        float q = a * r;
+        q = __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+        return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+    }
     /* x + u t for a hit, x + us / mu_t for a scattering; us is u or u s */
     static __device__ __forceinline__ float advance(float x, float us, bool hit, float t, float mu_t,
-                                                    float)
+                                                    float rmu_t)
     {
-        return x + (hit ? us * t : us / mu_t);
+        return x + (hit ? us * t : div_r(us, mu_t, rmu_t));
     }
     static __device__ __forceinline__ float sqrt(float x) { return sqrtf(x); }
     static __device__ __forceinline__ float rsqrt(float x) { return 1.0f / sqrtf(x); }
@@ -202,6 +222,17 @@ struct MathExact : FloatTable {
     static __device__ __forceinline__ float fmin(float a, float b) { return fminf(a, b); }
     static __device__ __forceinline__ float fabs(float x) { return fabsf(x); }
     static __device__ __forceinline__ float copysign(float a, float b) { return copysignf(a, b); }
+};
+
+/* The same with IEEE divisions, for voxel sizes and coefficients whose reciprocals, or
+ * the residuals of the quotients, leave FP32's normal range. */
+struct MathExactWide : MathExact {
+    static __device__ __forceinline__ float div_r(float a, float b, float) { return a / b; }
+    static __device__ __forceinline__ float advance(float x, float us, bool hit, float t, float mu_t,
+                                                    float)
+    {
+        return x + (hit ? us * t : us / mu_t);
+    }
 };
 
 /* Compiled only in a translation unit built with -use_fast_math, where the
@@ -242,7 +273,7 @@ struct MathFast : FloatTable {
 };
 
 /* FP64 stepping: the same loop with every transport quantity in double, the
- * coefficients derived in double from the table's float (mua, mus, g, n), and
+ * coefficients derived in double from the sets' float (mua, mus, g, n), and
  * the reference's double literals compared in double.  Random numbers stay the
  * reference's 32-bit draws.  Built with IEEE division and square root; the
  * precision reference for the FP32 policies. */
@@ -253,11 +284,20 @@ struct MathF64 {
     static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
     static __device__ __forceinline__ double mad(double a, double b, double c) { return a * b + c; }
     static __device__ __forceinline__ double div(double a, double b) { return a / b; }
-    static __device__ __forceinline__ double div_r(double a, double b, double) { return a / b; }
-    static __device__ __forceinline__ double advance(double x, double us, bool hit, double t,
-                                                     double mu_t, double)
+    /* a / b, correctly rounded, by r = 1 / b correctly rounded: the product with r and two
+     * corrections by the residual, which a fused multiply-add gives exactly (Markstein,
+     * IBM J. Res. Dev. 34, 1990: a quotient within one ulp becomes the nearest; the first
+     * correction brings it there).  5 instructions and no branch instead of about 16. */
+    static __device__ __forceinline__ double div_r(double a, double b, double r)
     {
-        return x + (hit ? us * t : us / mu_t);
+        double q = a * r;
+        q = __fma_rn(__fma_rn(-q, b, a), r, q);
+        return __fma_rn(__fma_rn(-q, b, a), r, q);
+    }
+    static __device__ __forceinline__ double advance(double x, double us, bool hit, double t,
+                                                     double mu_t, double rmu_t)
+    {
+        return x + (hit ? us * t : div_r(us, mu_t, rmu_t));
     }
     static __device__ __forceinline__ double sqrt(double x) { return ::sqrt(x); }
     static __device__ __forceinline__ double rsqrt(double x) { return 1.0 / ::sqrt(x); }
@@ -272,22 +312,27 @@ struct MathF64 {
     static __device__ __forceinline__ double fmin(double a, double b) { return ::fmin(a, b); }
     static __device__ __forceinline__ double fabs(double x) { return ::fabs(x); }
     static __device__ __forceinline__ double copysign(double a, double b) { return ::copysign(a, b); }
-    static __device__ __forceinline__ double n(const float4 *tt) { return tt[0].w; }
-    static __device__ __forceinline__ double mu_t(const float4 *tt)
+    using Geom = GeomDev64;
+    using Row = const double *; /* of the table in global memory, MC3D_TAB64_STRIDE a tissue */
+    static constexpr bool kShared = false;
+    static __device__ __forceinline__ Row row(Row tab, int tissue) { return tab + MC3D_TAB64_STRIDE * tissue; }
+    static __device__ __forceinline__ Row table(const KernelParams &P, const float4 *, int offset)
     {
-        return (double)tt[0].x + (double)tt[0].y;
+        return P.props64 + (offset / MC3D_TAB_STRIDE) * MC3D_TAB64_STRIDE;
     }
-    static __device__ __forceinline__ double albedo_c(const float4 *tt)
+    static __device__ __forceinline__ const Geom *geom(const KernelParams &P, const GeomDev *, int i)
     {
-        return mu_t(tt) > 0 ? (double)tt[0].x / mu_t(tt) : 0;
+        return P.geoms64 + i;
     }
-    static __device__ __forceinline__ double rmu_t(const float4 *tt) { return 1.0 / mu_t(tt); }
+    static __device__ __forceinline__ double mu_t(Row tt) { return tt[0]; }
+    static __device__ __forceinline__ double rmu_t(Row tt) { return tt[1]; }
+    static __device__ __forceinline__ double albedo_c(Row tt) { return tt[2]; }
+    static __device__ __forceinline__ double n(Row tt) { return tt[3]; }
     template <class M>
-    static __device__ __forceinline__ double hg_cos(const float4 *tt, double xi)
+    static __device__ __forceinline__ double hg_cos(Row tt, double xi)
     {
-        const double g = tt[0].z;
-        const double c = (1 - g * g) / (1 - g + 2 * g * xi);
-        return (1 + g * g - c * c) / (2 * g);
+        const double c = tt[4] / (tt[5] + tt[6] * xi);
+        return div_r(tt[7] - c * c, tt[6], tt[8]);
     }
     static __device__ __forceinline__ bool w_below_threshold(double w) { return w < 0.0001; }
     static __device__ __forceinline__ bool w_above_threshold(double w) { return w >= 0.0001; }
@@ -325,7 +370,6 @@ struct MathF64 {
 #define MC3D_NEAR_CRITICAL_F 0x1p-5f
 #define MC3D_NUM_PHOTON_STEPS 45
 #define MC3D_TISSUE_AIR 0
-#define MC3D_TAB_STRIDE 3 /* float4 per tissue in the optical table */
 
 
 /* 1 for a direction that moves up the axis (u >= 0), 0 for one that moves down */
@@ -343,9 +387,8 @@ static __device__ __forceinline__ R upward(R u)
  * rounded up, below the lower face (one voxel back).  Written as arithmetic on 0 and
  * 1: as predicates the three axes need more of them than a thread has. */
 template <class M, class R = typename M::real>
-static __device__ __forceinline__ R grid_index(R x, R up, float d_, float rd_)
+static __device__ __forceinline__ R grid_index(R x, R up, R d, R rd)
 {
-    const R d = d_, rd = rd_;
     const R fi = M::floor(M::div_r(x, d, rd));
     const R on_face = x == M::mul(fi + up, d) ? (R)1 : (R)0;
     const R below = x >= M::mul(fi, d) ? (R)0 : (R)1;
@@ -353,8 +396,8 @@ static __device__ __forceinline__ R grid_index(R x, R up, float d_, float rd_)
 }
 
 /* grid_index of the x and y axes */
-template <class M, class R = typename M::real>
-static __device__ __forceinline__ Pair<R> grid_index2(Pair<R> x, Pair<R> up, const GeomDev &g)
+template <class M, class G, class R = typename M::real>
+static __device__ __forceinline__ Pair<R> grid_index2(Pair<R> x, Pair<R> up, const G &g)
 {
     using Two = typename M::Pairs;
     using P2 = Pair<R>;
@@ -379,8 +422,8 @@ static __device__ __forceinline__ int cell_int(double f) { return f == f ? (int)
  * With JUMP the lookup reads the packed map (tissue | box radius << 8, one
  * 16-bit load), so the box radius rides in bits 8-15 of the result (0 above
  * the surface, where the tissue is air). */
-template <bool JUMP = false, class R = float>
-static __device__ __forceinline__ int tissue_at(const GeomDev &g, R fi, R fj, R fk, R z, R uz)
+template <bool JUMP = false, class G, class R>
+static __device__ __forceinline__ int tissue_at(const G &g, R fi, R fj, R fk, R z, R uz)
 {
     const int ci = min(max(cell_int(fi), 0), g.last_x);
     const int cj = min(max(cell_int(fj), 0), g.last_y);
@@ -402,17 +445,17 @@ static __device__ __forceinline__ int tissue_at(const GeomDev &g, R fi, R fj, R 
  * subtraction that follows, a photon lying exactly on a face would see its distance
  * to that face as the product's rounding error instead of 0. */
 template <class M, class R = typename M::real>
-static __device__ __forceinline__ R face_distance(R x, R u, R up, R fi, R r, float d, R *border)
+static __device__ __forceinline__ R face_distance(R x, R u, R up, R fi, R r, R d, R *border)
 {
     /* fi + r + 1 upward, fi - r downward (whole numbers: exact) */
-    *border = M::mul(fi + M::mad(up, M::mad((R)2, r, (R)1), -r), (R)d);
+    *border = M::mul(fi + M::mad(up, M::mad((R)2, r, (R)1), -r), d);
     return M::div(*border - x, u);
 }
 
 /* face_distance of the x and y axes */
-template <class M, class R = typename M::real>
+template <class M, class G, class R = typename M::real>
 static __device__ __forceinline__ Pair<R> face_distance2(Pair<R> x, Pair<R> u, Pair<R> up,
-                                                         Pair<R> fi, R r, const GeomDev &g,
+                                                         Pair<R> fi, R r, const G &g,
                                                          Pair<R> *border)
 {
     using Two = typename M::Pairs;
@@ -424,9 +467,8 @@ static __device__ __forceinline__ Pair<R> face_distance2(Pair<R> x, Pair<R> u, P
 
 /* src/mc3d_gpu.cu:113-126 */
 template <class M, class R = typename M::real>
-static __device__ __forceinline__ bool mirror(R *x, R *ux, float length_)
+static __device__ __forceinline__ bool mirror(R *x, R *ux, R length)
 {
-    const R length = length_;
     bool refl = (*x >= length) || (*x <= 0);
     *x = (*x >= length) ? 2 * length - *x : *x;
     *x = (*x <= 0) ? M::fabs(*x) : *x;
@@ -467,7 +509,7 @@ struct Spin {
 };
 
 template <class M, bool SPLIT_SIN2, class R = typename M::real>
-static __device__ __forceinline__ Spin<R> scatter(const float4 *tt, const PhotonT<R> &p,
+static __device__ __forceinline__ Spin<R> scatter(typename M::Row tt, const PhotonT<R> &p,
                                                   uint32_t e_hg, uint32_t e_phi)
 {
     Spin<R> o;
@@ -512,14 +554,14 @@ static __device__ __forceinline__ Spin<R> scatter(const float4 *tt, const Photon
  * part of the weight the reference loses. */
 template <class M, bool AMAP, bool JUMP = false, bool SPLIT_SIN2 = false,
           class R = typename M::real>
-static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float4 *tab,
+static __device__ __forceinline__ bool photon_step(const typename M::Geom &g, typename M::Row tab,
                                                    PhotonT<R> &p, uint64_t &rx, uint32_t ra,
                                                    const Acc &acc, R *db_out,
                                                    unsigned long long *amap, bool *lat_mirror)
 {
     /* per tissue: (mua, mus, g, n), (mu_t, 1/mu_t, mua/mu_t, 1/(2g)),
      * (1-g^2, 1-g, 2g, 1+g^2) -- each the float the reference computes per step */
-    const float4 *tt = tab + MC3D_TAB_STRIDE * (JUMP ? (p.tissue & 0xff) : p.tissue);
+    const typename M::Row tt = M::row(tab, JUMP ? (p.tissue & 0xff) : p.tissue);
     const R mu_t = M::mu_t(tt);
 
     /* the box's nearest face, src/mc3d_gpu.cu:29-49 */
@@ -612,9 +654,9 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
         bool redo = steep | (least_u < zero_thresh); /* the normalisation anew */
         const bool lateral = !(newx > 0) | !(newx < g.Lx) | !(newy > 0) | !(newy < g.Ly);
         if (((next_tissue ^ p.tissue) & 0xff) != 0 &&
-            M::n(tt) != M::n(tab + MC3D_TAB_STRIDE * (next_tissue & 0xff))) {
+            M::n(tt) != M::n(M::row(tab, next_tissue & 0xff))) {
             /* Fresnel, src/mc3d_gpu.cu:226-257 */
-            const R ni = M::n(tt), nt = M::n(tab + MC3D_TAB_STRIDE * (next_tissue & 0xff));
+            const R ni = M::n(tt), nt = M::n(M::row(tab, next_tissue & 0xff));
             const bool mx = p.i != nexti, my = p.j != nextj, mz = p.k != nextk;
             R cos_ai = mx ? p.ux : (my ? p.uy : p.uz);
             cos_ai = M::fabs(cos_ai);
@@ -701,7 +743,7 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
                 p.s = hit ? s : p.s - p.s;
                 *lat_mirror = false;
                 if (!refl && !(p.x > 0 && p.x < g.Lx && p.y > 0 && p.y < g.Ly))
-                    *lat_mirror = mirror<M>(&p.x, &p.ux, g.Lx) || mirror<M>(&p.y, &p.uy, g.Ly);
+                    *lat_mirror = mirror<M>(&p.x, &p.ux, (R)g.Lx) || mirror<M>(&p.y, &p.uy, (R)g.Ly);
                 return true;
             }
             if (!(W > 0)) { /* NaN weight: no free path, -log(1) */
@@ -764,7 +806,7 @@ static __device__ __forceinline__ bool photon_step(const GeomDev &g, const float
 /* i, j, k and tissue from the position, as at the start of every launch of
  * photontrack_step (src/mc3d_gpu.cu:168-171). */
 template <class M, bool JUMP = false, class R = typename M::real>
-static __device__ __forceinline__ void derive_cell(const GeomDev &g, PhotonT<R> &p)
+static __device__ __forceinline__ void derive_cell(const typename M::Geom &g, PhotonT<R> &p)
 {
     p.i = grid_index<M>(p.x, upward(p.ux), g.dx, g.rdx);
     p.j = grid_index<M>(p.y, upward(p.uy), g.dy, g.rdy);
@@ -776,8 +818,8 @@ static __device__ __forceinline__ void derive_cell(const GeomDev &g, PhotonT<R> 
  * every axis: strictly inside, or on the lower face moving up, or on the upper face
  * moving down.  Then re-deriving the cell and tissue at a launch boundary changes
  * nothing (above the surface the air rule would apply, which needs z > 0 here). */
-template <class R>
-static __device__ __forceinline__ bool cell_consistent(const GeomDev &g, const PhotonT<R> &p)
+template <class R, class G>
+static __device__ __forceinline__ bool cell_consistent(const G &g, const PhotonT<R> &p)
 {
     const R xl = p.i * (R)g.dx, xh = (p.i + (R)1) * (R)g.dx;
     const R yl = p.j * (R)g.dy, yh = (p.j + (R)1) * (R)g.dy;
@@ -800,7 +842,7 @@ static __device__ __forceinline__ bool finite_state(const PhotonT<R> &p)
  * face of its voxel and moves out through it, which happens when a scattering
  * move rounds onto a voxel face and the new direction points back across it. */
 template <class M, class R = typename M::real>
-static __device__ __forceinline__ R voxel_db(const GeomDev &g, const PhotonT<R> &p)
+static __device__ __forceinline__ R voxel_db(const typename M::Geom &g, const PhotonT<R> &p)
 {
     R b;
     const R t_x = face_distance<M>(p.x, p.ux, upward(p.ux), p.i, (R)0, g.dx, &b);
@@ -828,11 +870,11 @@ static __device__ __forceinline__ bool quickfix(PhotonT<R> &p, bool zero_db)
  * They change nothing but the mirror (which flips u while the photon sits on a
  * lateral face) and the boundary distance the quickfix looks at. */
 template <class M, class R = typename M::real>
-static __device__ __forceinline__ R masked_steps(const GeomDev &g, PhotonT<R> &p, int masked, R db)
+static __device__ __forceinline__ R masked_steps(const typename M::Geom &g, PhotonT<R> &p, int masked, R db)
 {
     for (int t = 0; t < masked; t++) {
         db = voxel_db<M>(g, p);
-        if (!mirror<M>(&p.x, &p.ux, g.Lx)) mirror<M>(&p.y, &p.uy, g.Ly);
+        if (!mirror<M>(&p.x, &p.ux, (R)g.Lx)) mirror<M>(&p.y, &p.uy, (R)g.Ly);
     }
     return db;
 }
@@ -931,9 +973,10 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
     extern __shared__ float4 sh_base[];
     unsigned long long *sh_rows = reinterpret_cast<unsigned long long *>(sh_base);
     float4 *sh_tab = reinterpret_cast<float4 *>(sh_rows + MC3D_THREAD_WORDS * blockDim.x);
-    for (int t = threadIdx.x; t < P.props_entries; t += blockDim.x) sh_tab[t] = P.props_table[t];
+    for (int t = threadIdx.x; M::kShared && t < P.props_entries; t += blockDim.x)
+        sh_tab[t] = P.props_table[t];
     GeomDev *sh_geom = reinterpret_cast<GeomDev *>(sh_tab + P.props_entries);
-    if (!ONE_GEOM)
+    if (M::kShared && !ONE_GEOM)
         for (int t = threadIdx.x; t < P.ngeoms; t += blockDim.x) sh_geom[t] = P.geoms[t];
     const Acc acc{sh_rows + MC3D_THREAD_WORDS * threadIdx.x};
     acc_clear(acc);
@@ -943,8 +986,20 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
     __syncthreads();
 
     int job = -1;
-    const GeomDev *gp = sh_geom;
-    const float4 *tab = sh_tab;
+    unsigned long long *amap = nullptr;
+    const typename M::Geom *gp = nullptr;
+    typename M::Row tab = nullptr;
+    /* the photon's geometry: the launch's only one from the kernel parameters */
+    auto geometry = [&]() -> const typename M::Geom & {
+        if constexpr (ONE_GEOM) return P.geom0;
+        else return *gp;
+    };
+    auto set_job = [&](int j) {
+        job = j;
+        gp = M::geom(P, sh_geom, P.jobs[job].geom);
+        tab = M::table(P, sh_tab, P.jobs[job].props_offset);
+        if (AMAP) amap = P.amap + P.jobs[job].amap_offset;
+    };
     int64_t &left = acc.left(), &local = acc.local();
     left = 0;
     uint64_t rx = 0;
@@ -953,7 +1008,6 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
     bool alive = false;
     bool drained = false; /* no stream left to take */
     int psteps = 0; /* steps of the photon before its present chunk */
-    unsigned long long *amap = nullptr;
     /* a lane without photons left in its stream takes the next stream */
     auto take_stream = [&]() {
         if (!alive && !drained) {
@@ -967,11 +1021,8 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
                 /* the per-thread tallies are the job's: flushed when the job changes */
                 if (job >= 0 && next_job != job)
                     acc_flush(acc, job_totals(P, job));
-                job = next_job;
+                set_job(next_job);
                 const JobDev &jb = P.jobs[job];
-                gp = sh_geom + jb.geom;
-                tab = sh_tab + jb.props_offset;
-                if (AMAP) amap = P.amap + jb.amap_offset;
                 local = gs - jb.stream_base + jb.stream_first;
                 left = jb.per_stream + (local < jb.remainder ? 1 : 0);
                 ra = stream_multiplier(P, local);
@@ -982,7 +1033,7 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
     /* a lane without a photon starts the next of its stream */
     auto start_photon = [&]() {
         if (!alive && left != 0) {
-            const GeomDev &g = ONE_GEOM ? P.geom0 : *gp;
+            const auto &g = geometry();
             /* photontrack_reinitialize, src/mc3d_gpu.cu:74-111 */
             if (P.jobs[job].beam == 0) {
                 p.x = (R)g.Lx * (R)mc3d_rand_co(&rx, ra);
@@ -994,7 +1045,7 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
             p.z = 0;
             p.ux = 0; p.uy = 0; p.uz = 1;
             /* specular reflection from air into tissue type 1 (src/mc3d_gpu.cu:67-70, 500) */
-            const R n0 = M::n(tab + MC3D_TAB_STRIDE * MC3D_TISSUE_AIR), n1 = M::n(tab + MC3D_TAB_STRIDE);
+            const R n0 = M::n(M::row(tab, MC3D_TISSUE_AIR)), n1 = M::n(M::row(tab, 1));
             const R rsp = M::div(n0 - n1, n0 + n1);
             p.W = M::mad(-rsp, rsp, (R)1);
             p.s = -M::log((R)mc3d_rand_oc(&rx, ra));
@@ -1011,7 +1062,7 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
      * loop early runs on alone, and from then on the warp steps in pieces (4.7 lanes a
      * chunk's end instead of 32, layered 1e6 photons). */
     auto run_chunk = [&]() {
-        const GeomDev &g = ONE_GEOM ? P.geom0 : *gp;
+        const auto &g = geometry();
         /* The chunk's steps, fewer where the step cap comes first.  Merged steps: the
          * quickfix must see the boundary distance of the reference's one-voxel DDA
          * for the chunk's last step, not the merged box's (which is never 0 inside a
@@ -1099,7 +1150,7 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
             }
             acc[slot] += q;
             /* the launch weight 1 - Rsp again, as at the photon's start */
-            const R n0 = M::n(tab + MC3D_TAB_STRIDE * MC3D_TISSUE_AIR), n1 = M::n(tab + MC3D_TAB_STRIDE);
+            const R n0 = M::n(M::row(tab, MC3D_TISSUE_AIR)), n1 = M::n(M::row(tab, 1));
             const R rsp = M::div(n0 - n1, n0 + n1);
             const uint64_t qw0 = M::qw(M::mad(-rsp, rsp, (R)1));
             acc[T_W_LAUNCHED] += qw0;
@@ -1171,10 +1222,7 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
                 p.tissue = q.tissue;
                 ra = q.ra;
                 psteps = q.psteps;
-                job = q.job;
-                gp = sh_geom + P.jobs[job].geom;
-                tab = sh_tab + P.jobs[job].props_offset;
-                if (AMAP) amap = P.amap + P.jobs[job].amap_offset;
+                set_job(q.job);
             } else {
                 left = 0;
             }

@@ -4,7 +4,11 @@
  * quantity is a double; the loop, its quirks and the random numbers are those of
  * the FP32 kernels, with one step per voxel face or merged steps (the step mode
  * of the plan).  It is the precision reference the FP32 results are stated
- * against.
+ * against.  What is constant per tissue or geometry comes in double from two tables
+ * (GeomDev64, KernelParams::props64), and divisions by it are done through its
+ * reciprocal (MathF64::div_r): 2e5 layered photons took 48.4 ms with 14 divisions and 13
+ * conversions a step, 35.5 ms with 6.  128 registers, 16 warps an SM: 140 (12 warps)
+ * spill nothing but took 88 ms instead of 82 for 1e6 photons.
  */
 #include "mc3d_engine.cuh"
 #include "mc3d_launch.h"

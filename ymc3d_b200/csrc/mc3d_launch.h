@@ -18,6 +18,8 @@ namespace mc3d {
 #define MC3D_VARIANT_VOXEL_STEPS 2
 /* one geometry in the launch: its descriptor is read from the kernel parameters */
 #define MC3D_VARIANT_ONE_GEOM 4
+/* exact math with IEEE divisions by voxel sizes and mu_t (outside [2^-60, 2^60]) */
+#define MC3D_VARIANT_DIVIDE 8
 
 /* dynamic shared memory of a photon kernel: the threads' rows, optical tables, geometry
  * descriptors */
@@ -30,14 +32,14 @@ static inline size_t photon_smem(int props_entries, int ngeoms, int block)
 cudaError_t launch_photon_fast(const KernelParams &P, int grid, int block, size_t smem,
                                cudaStream_t stream, int variant);
 cudaError_t launch_photon_exact(const KernelParams &P, int grid, int block, size_t smem,
-                                cudaStream_t stream);
+                                cudaStream_t stream, int variant);
 cudaError_t launch_photon_f64(const KernelParams &P, int grid, int block, size_t smem,
                               cudaStream_t stream, int variant);
 cudaError_t occupancy_photon_fast(int block, size_t smem, int *blocks_per_sm, int variant);
 cudaError_t occupancy_photon_f64(int block, size_t smem, int *blocks_per_sm, int variant);
 cudaError_t smem_limit_photon_f64(size_t smem);
 cudaError_t attributes_photon_f64(cudaFuncAttributes *attr);
-cudaError_t occupancy_photon_exact(int block, size_t smem, int *blocks_per_sm);
+cudaError_t occupancy_photon_exact(int block, size_t smem, int *blocks_per_sm, int variant);
 cudaError_t smem_limit_photon_fast(size_t smem);
 cudaError_t smem_limit_photon_exact(size_t smem);
 cudaError_t attributes_photon_fast(cudaFuncAttributes *attr);
