@@ -57,14 +57,20 @@ struct Pair {
 template <class M, class R>
 struct PairwiseOps {
     using P2 = Pair<R>;
-    static __device__ __forceinline__ P2 mul(P2 x, P2 y) { return {M::mul(x.a, y.a), M::mul(x.b, y.b)}; }
+    static __device__ __forceinline__ P2 mul(P2 x, P2 y)
+    {
+        return {M::mul(x.a, y.a), M::mul(x.b, y.b)};
+    }
     static __device__ __forceinline__ P2 add(P2 x, P2 y) { return {x.a + y.a, x.b + y.b}; }
     static __device__ __forceinline__ P2 sub(P2 x, P2 y) { return {x.a - y.a, x.b - y.b}; }
     static __device__ __forceinline__ P2 mad(P2 x, P2 y, P2 z)
     {
         return {M::mad(x.a, y.a, z.a), M::mad(x.b, y.b, z.b)};
     }
-    static __device__ __forceinline__ P2 div(P2 x, P2 y) { return {M::div(x.a, y.a), M::div(x.b, y.b)}; }
+    static __device__ __forceinline__ P2 div(P2 x, P2 y)
+    {
+        return {M::div(x.a, y.a), M::div(x.b, y.b)};
+    }
     static __device__ __forceinline__ P2 div_r(P2 x, P2 y, P2 r)
     {
         return {M::div_r(x.a, y.a, r.a), M::div_r(x.b, y.b, r.b)};
@@ -130,12 +136,13 @@ struct FloatTable {
     using Geom = GeomDev;
     using Row = const float4 *; /* of the table in shared memory, MC3D_TAB_STRIDE a tissue */
     static constexpr bool kShared = true; /* table and geometries are read from shared memory */
-    static __device__ __forceinline__ Row row(Row tab, int tissue) { return tab + MC3D_TAB_STRIDE * tissue; }
+    static __device__ __forceinline__ Row row(Row tab, int t) { return tab + MC3D_TAB_STRIDE * t; }
     static __device__ __forceinline__ Row table(const KernelParams &, Row shared, int offset)
     {
         return shared + offset;
     }
-    static __device__ __forceinline__ const Geom *geom(const KernelParams &, const GeomDev *shared, int i)
+    static __device__ __forceinline__ const Geom *geom(const KernelParams &, const GeomDev *shared,
+                                                       int i)
     {
         return shared + i;
     }
@@ -315,7 +322,7 @@ struct MathF64 {
     using Geom = GeomDev64;
     using Row = const double *; /* of the table in global memory, MC3D_TAB64_STRIDE a tissue */
     static constexpr bool kShared = false;
-    static __device__ __forceinline__ Row row(Row tab, int tissue) { return tab + MC3D_TAB64_STRIDE * tissue; }
+    static __device__ __forceinline__ Row row(Row tab, int t) { return tab + MC3D_TAB64_STRIDE * t; }
     static __device__ __forceinline__ Row table(const KernelParams &P, const float4 *, int offset)
     {
         return P.props64 + (offset / MC3D_TAB_STRIDE) * MC3D_TAB64_STRIDE;
@@ -552,13 +559,13 @@ static __device__ __forceinline__ Spin<R> scatter(typename M::Row tt, const Phot
  * coordinate that was not snapped rounded onto a face; the photon then takes
  * zero-length steps until the quickfix at its chunk's end removes it, which is
  * part of the weight the reference loses. */
-template <class M, bool AMAP, bool JUMP = false, bool SPLIT_SIN2 = false,
-          class R = typename M::real>
+template <class M, bool AMAP, bool JUMP, bool ONE_GEOM, class R = typename M::real>
 static __device__ __forceinline__ bool photon_step(const typename M::Geom &g, typename M::Row tab,
                                                    PhotonT<R> &p, uint64_t &rx, uint32_t ra,
                                                    const Acc &acc, R *db_out,
                                                    unsigned long long *amap, bool *lat_mirror)
 {
+    constexpr bool SPLIT_SIN2 = M::kFast && AMAP && JUMP && ONE_GEOM; /* see scatter */
     /* per tissue: (mua, mus, g, n), (mu_t, 1/mu_t, mua/mu_t, 1/(2g)),
      * (1-g^2, 1-g, 2g, 1+g^2) -- each the float the reference computes per step */
     const typename M::Row tt = M::row(tab, JUMP ? (p.tissue & 0xff) : p.tissue);
@@ -653,115 +660,122 @@ static __device__ __forceinline__ bool photon_step(const typename M::Geom &g, ty
         bool again = steep && !hit;   /* the scattering anew */
         bool redo = steep | (least_u < zero_thresh); /* the normalisation anew */
         const bool lateral = !(newx > 0) | !(newx < g.Lx) | !(newy > 0) | !(newy < g.Ly);
-        if (((next_tissue ^ p.tissue) & 0xff) != 0 &&
-            M::n(tt) != M::n(M::row(tab, next_tissue & 0xff))) {
-            /* Fresnel, src/mc3d_gpu.cu:226-257 */
-            const R ni = M::n(tt), nt = M::n(M::row(tab, next_tissue & 0xff));
-            const bool mx = p.i != nexti, my = p.j != nextj, mz = p.k != nextk;
-            R cos_ai = mx ? p.ux : (my ? p.uy : p.uz);
-            cos_ai = M::fabs(cos_ai);
-            cos_ai = (cos_ai > 1) ? 1 : cos_ai;
-            const R ni_nt = M::div(ni, nt);
-            /* sin(acos(c)); fast math evaluates it as sqrt((1 - c)(1 + c)), the same
-             * value without the polynomial of acosf (and more accurate near c = 1) */
-            const R sin_ai = M::kFast ? M::sqrt(M::mul((R)1 - cos_ai, (R)1 + cos_ai))
-                                      : M::sin(M::acos(cos_ai));
-            const R sin_at = M::mul(ni_nt, sin_ai);
-            R cos_at = M::sqrt(M::mad(-sin_at, sin_at, (R)1));
-            const R cs = M::mul(cos_ai, sin_at), cc = M::mul(cos_ai, cos_at);
-            const R R1 = M::div(M::mad(sin_ai, cos_at, -cs), M::mad(sin_ai, cos_at, cs));
-            const R R2 = M::div(M::mad(-sin_ai, sin_at, cc), M::mad(sin_at, sin_at, cc));
-            /* 0.5 is a double literal there too */
-            R Rf = 0.5 * R1 * R1 * M::mad(R2, R2, (R)1);
-            Rf = (sin_at > 1) ? 1 : Rf;
-            R lat = ni_nt; /* scale of the transmitted lateral cosines */
-            if (M::kFast && M::fabs(M::mad(-sin_at, sin_at, (R)1)) < MC3D_NEAR_CRITICAL_F) {
-                /* Near the critical angle 1 - sin_at^2 cancels in float and R is steep:
-                 * the same formulas in FP64, sin_ai from cos_ai directly, and the
-                 * transmitted direction renormalised in FP64. */
-                const double c = cos_ai;
-                const double rn = (double)ni / (double)nt;
-                const double si = sqrt((1.0 - c) * (1.0 + c));
-                const double st = rn * si;
-                const double ca = sqrt(fmax((1.0 - st) * (1.0 + st), 0.0));
-                const double R1 = (si * ca - c * st) / (si * ca + c * st);
-                const double R2 = (c * ca - si * st) / (c * ca + st * st);
-                Rf = (st >= 1.0) ? (R)1 : (R)(0.5 * R1 * R1 * (1.0 + R2 * R2));
-                const bool xa = mx;
-                const bool ya = !xa && my;
-                const bool za = !xa && !ya && mz;
-                const double ax = xa ? 0.0 : (double)p.ux;
-                const double ay = ya ? 0.0 : (double)p.uy;
-                const double az = za ? 0.0 : (double)p.uz;
-                const double lat2 = rn * rn * (ax * ax + ay * ay + az * az);
-                const double sc = 1.0 / sqrt(ca * ca + lat2);
-                cos_at = (R)(ca * sc);
-                lat = (R)(rn * sc);
-            }
-            /* The reflection is the step's first draw, so the other four are each one
-             * draw later than taken above. */
-            refl = mc3d_u32_to_float_rz(e_rr) * 0x1p-32f < Rf;
-            e_rr = e_hg;
-            e_hg = e_phi;
-            e_phi = e_s;
-            rx = mc3d_mwc_next(rx, ra);
-            e_s = (uint32_t)rx;
-            if (hit) {
-                const R tx = mx ? M::copysign(cos_at, M::mul(p.ux, cos_at)) : M::mul(p.ux, lat);
-                const R ty = (my && !mx) ? M::copysign(cos_at, M::mul(p.uy, cos_at))
-                                         : M::mul(p.uy, lat);
-                const R tz = (mz && !my && !mx) ? M::copysign(cos_at, M::mul(p.uz, cos_at))
-                                                : M::mul(p.uz, lat);
-                nux = refl ? (mx ? -p.ux : p.ux) : tx;
-                nuy = refl ? (my ? -p.uy : p.uy) : ty;
-                nuz = refl ? (mz ? -p.uz : p.uz) : tz;
-            }
-            again = !hit; /* an interaction that rounded onto the face */
-            redo = true;
-            acc[T_FRESNEL] += 1;
-        }
-        if (!M::w_above_threshold(W) | (mu_t == 0)) {
-            /* Russian roulette, src/mc3d_gpu.cu:275-277 */
-            if (M::w_below_threshold(W) && !hit && mu_t != 0) {
-                const float eps = mc3d_u32_to_float_rz(e_rr) * 0x1p-32f;
-                const R newW = (eps < MC3D_SURVIVAL_LT_F) ? M::roulette_survivor(W) : (R)0;
-                /* absorbed weight is booked at the photon's end as Q(W0) - Q(W_end) - lost;
-                 * a roulette event moves its share from there to the roulette tallies */
-                if (newW == 0) {
-                    uint64_t k = M::qw(W);
-                    acc[T_RR_KILLED] += k;
-                    acc[T_ABSORBED] -= k;
-                } else {
-                    uint64_t c = M::qw(newW) - M::qw(W);
-                    acc[T_RR_CREATED] += c;
-                    acc[T_ABSORBED] += c;
+        const bool low = !M::w_above_threshold(W) | (mu_t == 0);
+        /* Two of three lanes that come here only touch a lateral face: with one geometry
+         * they pass the three parts below at once (layered 1e6 22.4 -> 21.8 ms, pencil beam
+         * 1e6 18.6 -> 18.1).  Launches over several geometries, whose inclusions change the
+         * index in half of a warp's steps, lose by the extra test (22.5 -> 23.2 ms). */
+        if (!ONE_GEOM || (changed != 0) | low | redo) {
+            if (((next_tissue ^ p.tissue) & 0xff) != 0 &&
+                M::n(tt) != M::n(M::row(tab, next_tissue & 0xff))) {
+                /* Fresnel, src/mc3d_gpu.cu:226-257 */
+                const R ni = M::n(tt), nt = M::n(M::row(tab, next_tissue & 0xff));
+                const bool mx = p.i != nexti, my = p.j != nextj, mz = p.k != nextk;
+                R cos_ai = mx ? p.ux : (my ? p.uy : p.uz);
+                cos_ai = M::fabs(cos_ai);
+                cos_ai = (cos_ai > 1) ? 1 : cos_ai;
+                const R ni_nt = M::div(ni, nt);
+                /* sin(acos(c)); fast math evaluates it as sqrt((1 - c)(1 + c)), the same
+                 * value without the polynomial of acosf (and more accurate near c = 1) */
+                const R sin_ai = M::kFast ? M::sqrt(M::mul((R)1 - cos_ai, (R)1 + cos_ai))
+                                          : M::sin(M::acos(cos_ai));
+                const R sin_at = M::mul(ni_nt, sin_ai);
+                R cos_at = M::sqrt(M::mad(-sin_at, sin_at, (R)1));
+                const R cs = M::mul(cos_ai, sin_at), cc = M::mul(cos_ai, cos_at);
+                const R R1 = M::div(M::mad(sin_ai, cos_at, -cs), M::mad(sin_ai, cos_at, cs));
+                const R R2 = M::div(M::mad(-sin_ai, sin_at, cc), M::mad(sin_at, sin_at, cc));
+                /* 0.5 is a double literal there too */
+                R Rf = 0.5 * R1 * R1 * M::mad(R2, R2, (R)1);
+                Rf = (sin_at > 1) ? 1 : Rf;
+                R lat = ni_nt; /* scale of the transmitted lateral cosines */
+                if (M::kFast && M::fabs(M::mad(-sin_at, sin_at, (R)1)) < MC3D_NEAR_CRITICAL_F) {
+                    /* Near the critical angle 1 - sin_at^2 cancels in float and R is steep:
+                     * the same formulas in FP64, sin_ai from cos_ai directly, and the
+                     * transmitted direction renormalised in FP64. */
+                    const double c = cos_ai;
+                    const double rn = (double)ni / (double)nt;
+                    const double si = sqrt((1.0 - c) * (1.0 + c));
+                    const double st = rn * si;
+                    const double ca = sqrt(fmax((1.0 - st) * (1.0 + st), 0.0));
+                    const double R1 = (si * ca - c * st) / (si * ca + c * st);
+                    const double R2 = (c * ca - si * st) / (c * ca + st * st);
+                    Rf = (st >= 1.0) ? (R)1 : (R)(0.5 * R1 * R1 * (1.0 + R2 * R2));
+                    const bool xa = mx;
+                    const bool ya = !xa && my;
+                    const bool za = !xa && !ya && mz;
+                    const double ax = xa ? 0.0 : (double)p.ux;
+                    const double ay = ya ? 0.0 : (double)p.uy;
+                    const double az = za ? 0.0 : (double)p.uz;
+                    const double lat2 = rn * rn * (ax * ax + ay * ay + az * az);
+                    const double sc = 1.0 / sqrt(ca * ca + lat2);
+                    cos_at = (R)(ca * sc);
+                    lat = (R)(rn * sc);
                 }
-                W = newW;
-            }
-            if (W <= 0 || mu_t == 0) { /* freeze (:303-311): the photon stays where it is */
-                p.W = W;
-                p.s = hit ? s : p.s - p.s;
-                *lat_mirror = false;
-                if (!refl && !(p.x > 0 && p.x < g.Lx && p.y > 0 && p.y < g.Ly))
-                    *lat_mirror = mirror<M>(&p.x, &p.ux, (R)g.Lx) || mirror<M>(&p.y, &p.uy, (R)g.Ly);
-                return true;
-            }
-            if (!(W > 0)) { /* NaN weight: no free path, -log(1) */
-                e_s = 0;
+                /* The reflection is the step's first draw, so the other four are each one
+                 * draw later than taken above. */
+                refl = mc3d_u32_to_float_rz(e_rr) * 0x1p-32f < Rf;
+                e_rr = e_hg;
+                e_hg = e_phi;
+                e_phi = e_s;
+                rx = mc3d_mwc_next(rx, ra);
+                e_s = (uint32_t)rx;
+                if (hit) {
+                    const R tx = mx ? M::copysign(cos_at, M::mul(p.ux, cos_at)) : M::mul(p.ux, lat);
+                    const R ty = (my && !mx) ? M::copysign(cos_at, M::mul(p.uy, cos_at))
+                                             : M::mul(p.uy, lat);
+                    const R tz = (mz && !my && !mx) ? M::copysign(cos_at, M::mul(p.uz, cos_at))
+                                                    : M::mul(p.uz, lat);
+                    nux = refl ? (mx ? -p.ux : p.ux) : tx;
+                    nuy = refl ? (my ? -p.uy : p.uy) : ty;
+                    nuz = refl ? (mz ? -p.uz : p.uz) : tz;
+                }
+                again = !hit; /* an interaction that rounded onto the face */
                 redo = true;
+                acc[T_FRESNEL] += 1;
             }
-        }
-        if (redo) {
-            if (again) {
-                const Spin<R> sp = scatter<M, SPLIT_SIN2>(tt, p, e_hg, e_phi);
-                nux = steep ? M::mul(sp.sintheta, sp.cosphi) : sp.ux;
-                nuy = steep ? M::mul(sp.sintheta, sp.sinphi) : sp.uy;
-                nuz = steep ? M::copysign(sp.costheta, M::mul(sp.costheta, p.uz)) : sp.uz;
+            if (low) {
+                /* Russian roulette, src/mc3d_gpu.cu:275-277 */
+                if (M::w_below_threshold(W) && !hit && mu_t != 0) {
+                    const float eps = mc3d_u32_to_float_rz(e_rr) * 0x1p-32f;
+                    const R newW = (eps < MC3D_SURVIVAL_LT_F) ? M::roulette_survivor(W) : (R)0;
+                    /* absorbed weight is booked at the photon's end as Q(W0) - Q(W_end) - lost;
+                     * a roulette event moves its share from there to the roulette tallies */
+                    if (newW == 0) {
+                        uint64_t k = M::qw(W);
+                        acc[T_RR_KILLED] += k;
+                        acc[T_ABSORBED] -= k;
+                    } else {
+                        uint64_t c = M::qw(newW) - M::qw(W);
+                        acc[T_RR_CREATED] += c;
+                        acc[T_ABSORBED] += c;
+                    }
+                    W = newW;
+                }
+                if (W <= 0 || mu_t == 0) { /* freeze (:303-311): the photon stays where it is */
+                    p.W = W;
+                    p.s = hit ? s : p.s - p.s;
+                    *lat_mirror = false;
+                    if (!refl && !(p.x > 0 && p.x < g.Lx && p.y > 0 && p.y < g.Ly))
+                        *lat_mirror = mirror<M>(&p.x, &p.ux, (R)g.Lx) || mirror<M>(&p.y, &p.uy, (R)g.Ly);
+                    return true;
+                }
+                if (!(W > 0)) { /* NaN weight: no free path, -log(1) */
+                    e_s = 0;
+                    redo = true;
+                }
             }
-            nux = (M::fabs(nux) < zero_thresh) ? 0 : nux;
-            nuy = (M::fabs(nuy) < zero_thresh) ? 0 : nuy;
-            nuz = (M::fabs(nuz) < zero_thresh) ? 0 : nuz;
-            if (M::kFast) finish();
+            if (redo) {
+                if (again) {
+                    const Spin<R> sp = scatter<M, SPLIT_SIN2>(tt, p, e_hg, e_phi);
+                    nux = steep ? M::mul(sp.sintheta, sp.cosphi) : sp.ux;
+                    nuy = steep ? M::mul(sp.sintheta, sp.sinphi) : sp.uy;
+                    nuz = steep ? M::copysign(sp.costheta, M::mul(sp.costheta, p.uz)) : sp.uz;
+                }
+                nux = (M::fabs(nux) < zero_thresh) ? 0 : nux;
+                nuy = (M::fabs(nuy) < zero_thresh) ? 0 : nuy;
+                nuz = (M::fabs(nuz) < zero_thresh) ? 0 : nuz;
+                if (M::kFast) finish();
+            }
         }
         /* The mirrors, short-circuited as in src/mc3d_gpu.cu:330, both axes at once.  A
          * mirror turns its component before or after the normalisation, which keeps the
@@ -1078,8 +1092,8 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
         bool vzero = false;
         for (;;) {
             while (!froze && chunk < stop) {
-                froze = photon_step<M, AMAP, JUMP, M::kFast && AMAP && JUMP && ONE_GEOM>(
-                    g, tab, p, rx, ra, acc, &db, amap, &lat_mirror);
+                froze = photon_step<M, AMAP, JUMP, ONE_GEOM>(g, tab, p, rx, ra, acc, &db, amap,
+                                                             &lat_mirror);
                 chunk++;
             }
             if (!JUMP || froze || stop == cap) break;

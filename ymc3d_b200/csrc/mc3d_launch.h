@@ -11,10 +11,7 @@
 
 namespace mc3d {
 
-/* fast kernel variant bits: one step per voxel face instead of merged steps.
- * (A 64-register build of 4 blocks of 256 per SM measured 2-12 % slower than the
- * 80-register one and is not built: one kernel serves every launch shape, so the
- * tallies cannot depend on the shape.) */
+/* kernel variant bits: one step per voxel face instead of merged steps */
 #define MC3D_VARIANT_VOXEL_STEPS 2
 /* one geometry in the launch: its descriptor is read from the kernel parameters */
 #define MC3D_VARIANT_ONE_GEOM 4
