@@ -43,11 +43,10 @@ OPS_STEP, SFU_STEP = 152, 20
 OPS_JUMP = 8
 OPS_FRESNEL, SFU_FRESNEL = 37, 6
 FP32_LANES_PER_SM, SFU_LANES_PER_SM = 128, 16
-# DRAM bytes read + written by one photon-kernel launch of the layered workload
-# (ncu dram__bytes_read.sum + dram__bytes_write.sum = 30,852,096 + 0 on a
-# 1e7-photon launch): the first touch of grid, packed cell map, table and tallies,
-# independent of the photon count
-TRAFFIC_BYTES_PER_LAUNCH = 30_852_096
+# DRAM bytes read + written by one photon-kernel launch of the layered workload (ncu
+# dram__bytes_read.sum + dram__bytes_write.sum = 114.0e6 + 4.1e6 on a 1e7-photon launch): the
+# first touch of grid, packed cell map, table and tallies, and 8 bytes of stream state a photon
+TRAFFIC_BYTES_PER_LAUNCH, TRAFFIC_BYTES_PER_PHOTON = 38_100_000, 8
 
 
 def parse():
@@ -324,7 +323,7 @@ def run_ours(args):
     fp32_ops = steps_per_s * (ops_step - SFU_STEP) + fres_per_s * (OPS_FRESNEL - SFU_FRESNEL)
     sfu_peak = sms * SFU_LANES_PER_SM * f_max
     fp32_peak = sms * FP32_LANES_PER_SM * f_max
-    traffic = TRAFFIC_BYTES_PER_LAUNCH
+    traffic = TRAFFIC_BYTES_PER_LAUNCH + TRAFFIC_BYTES_PER_PHOTON * (int(photons_step) // world)
     block, grid, smem = plan.shape()
     line = {
         "metric": "photons/s (layered tissue + vessel, 256x256x128, uniform beam, 1 B200)",

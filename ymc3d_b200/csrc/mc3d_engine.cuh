@@ -545,7 +545,7 @@ static __device__ __forceinline__ Spin<R> scatter(typename M::Row tt, const Phot
  * step's box is the cube of voxels within Chebyshev distance r of the photon's
  * voxel.  The box holds only the photon's tissue, and a shell of one voxel around
  * it has the photon's refractive index and stays clear of the top and lateral
- * faces (pack_kernel): a step that reaches a box face crosses into a voxel of the
+ * faces (cell_of): a step that reaches a box face crosses into a voxel of the
  * same index, with no Fresnel event, no mirror and no air rule, exactly as the
  * reference's step at that face would (snapped, next voxel by the face rule; that
  * voxel may hold another tissue of the same index, whose coefficients the next
@@ -558,7 +558,11 @@ static __device__ __forceinline__ Spin<R> scatter(typename M::Row tt, const Phot
  * (src/mc3d_gpu.cu:334-339).  That rule can leave the index one voxel off when a
  * coordinate that was not snapped rounded onto a face; the photon then takes
  * zero-length steps until the quickfix at its chunk's end removes it, which is
- * part of the weight the reference loses. */
+ * part of the weight the reference loses.
+ *
+ * Bound by instruction issue, so the straight line holds what most lanes do and all else
+ * stands behind one test: 188 thread-instructions a merged step (283 when every rule had
+ * its own branch), layered 1e7 photons 221.7 -> 163.4 ms. */
 template <class M, bool AMAP, bool JUMP, bool ONE_GEOM, class R = typename M::real>
 static __device__ __forceinline__ bool photon_step(const typename M::Geom &g, typename M::Row tab,
                                                    PhotonT<R> &p, uint64_t &rx, uint32_t ra,

@@ -8,10 +8,16 @@
 
 namespace mc3d {
 
-/* 96 registers: 20 warps an SM in blocks of 128 threads, and no spills.  80 registers
- * (24 warps) spill 120 bytes a step, 104 (16 warps) hide less: 1e7 layered photons took
- * 174.4 ms with 80, 175.5 with 96 and 184.5 with 104, 2e5 skin-model photons 4.59, 3.97
- * and 3.59 ms, because a photon's own steps come slower the more warps share an SM.
+/* What bounds them: instruction issue while streams last (80 % of slots; 188
+ * thread-instructions a merged step, 283 at first), the fixed latencies of a lone photon's
+ * step at a launch's end (0.30 us, 0.62 at first).  1e7 layered photons 221.7 -> 163.4 ms,
+ * 1e4 in a pencil beam 11.3 -> 5.4 ms, one step per face (1e6) 180 -> 101 ms.
+ *
+ * 96 registers: 20 warps an SM in blocks of 128 threads, and no spills with one geometry.
+ * 80 registers (24 warps) spill 224 bytes: 2.7 % faster on 1e7 layered photons (163.9
+ * against 168.3 ms), 5 % slower on twelve mixed geometries and on the grid beyond L2, and a
+ * photon's own steps come slower the more warps share an SM (2e5 skin-model photons 4.59
+ * against 3.97 ms).  104 registers (16 warps) hide less: 7 % slower on 1e7.
  *
  * Eight instantiations: merged steps (box DDA over uniform cubes) or one step
  * per voxel face; with or without the absorption map; several geometries (their
