@@ -171,3 +171,57 @@ def test_exact_divisions_at_the_range_ends(table, scale, absorption):
     o = oracle_job(g, p, job, table, photon_log=True, max_steps=20_000)
     assert np.array_equal(_log(r), o["photon_log"].view(np.uint8).reshape(600, -1))
     assert r.totals == o["totals"] and np.array_equal(r.drs, o["drs"])
+
+
+# A grid with more than 2^21 voxels along an axis takes the kernels without the short
+# index arithmetic, and takes the launch's other jobs with it.
+@pytest.mark.parametrize("steps,absorption", [("merged", False), ("merged", True),
+                                              ("voxel", False), ("voxel", True)])
+def test_long_axis_kernels_agree(table, steps, absorption):
+    rng = np.random.default_rng(5)
+    geo = lambda t: m.Geometry(np.ascontiguousarray(t), 0.05, 0.04, 0.06)
+    t = np.kron(rng.integers(1, 4, (3, 4, 5)), np.ones((9, 7, 8), int)).astype(np.uint8)
+    t[:2, :3, :3] = 0
+    p = m.OpticalProps.from_tissues([(0.3, 9.0, 0.9, 1.4), (2.0, 20.0, 0.7, 1.33),
+                                     (0.1, 4.0, 0.0, 1.5)])
+    job = m.Job(0, 0, 30_000, 99, "uniform")
+    long = np.ones((1, 1, (1 << 21) + 1), np.uint8)
+    runs = []
+    for last in (long[:, :, :-1], long):
+        runs.append(m.run([geo(t), geo(last)], [p], [job, m.Job(1, 0, 2_000, 7, "pencil")],
+                          table=table, steps=steps, absorption_map=absorption, photon_log=True))
+    (a, _), (b, w) = runs
+    assert np.array_equal(_log(a), _log(b)) and a.totals == b.totals
+    assert np.array_equal(a.drs, b.drs) and np.array_equal(a.trans, b.trans)
+    alone = m.run([geo(long)], [p], [m.Job(0, 0, 2_000, 7, "pencil")], table=table, steps=steps,
+                  absorption_map=absorption, photon_log=True)[0]
+    assert residual(w.totals) == 0 and residual(alone.totals) == 0
+    if absorption:
+        assert np.array_equal(a.absorption, b.absorption)
+        assert int(alone.absorption.sum()) == alone.totals["absorbed"]
+    else:
+        assert np.array_equal(_log(w), _log(alone)) and w.totals == alone.totals
+
+
+def test_long_axis_noalloc(table):
+    """the allocation-free entry's kernel for such a grid against mc3d_run's"""
+    import ctypes as C
+
+    import torch
+
+    t = np.ones((1, 1, (1 << 21) + 1), np.uint8)
+    g, p = m.Geometry(t, 0.05, 0.04, 0.06), m.OpticalProps.from_tissues([(0.3, 9.0, 0.9, 1.4)])
+    job = m.Job(0, 0, 2_000, 7, "uniform")
+    tab = np.ascontiguousarray(table[:100_001])
+    ref = m.run([g], [p], [job], table=tab, steps="voxel")[0]
+    dev = torch.device("cuda", 0)
+    tissue = torch.from_numpy(t.reshape(-1).copy()).to(dev)
+    outs = [torch.zeros(t.size, dtype=torch.int64, device=dev) for _ in range(3)]
+    totals = torch.zeros(14, dtype=torch.int64, device=dev)
+    cg, cp, cj = m.CGeom(t.size, 1, 1, 0, g.dx, g.dy, g.dz, tissue.data_ptr()), p.c(), job.c()
+    assert m.lib().mc3d_run_noalloc(C.byref(cg), C.byref(cp), C.byref(cj), tab.ctypes.data,
+                                    len(tab), 0, None, *[o.data_ptr() for o in outs],
+                                    totals.data_ptr()) == 0
+    torch.cuda.synchronize(dev)
+    assert list(ref.totals.values()) == totals.tolist()
+    assert np.array_equal(outs[0].cpu().numpy().view(np.uint64), ref.drs.reshape(-1))

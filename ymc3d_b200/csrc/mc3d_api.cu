@@ -736,6 +736,7 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
                                               : smem_limit_photon_f64(max_dyn));
     }
     p->variant = (p->jump ? 0 : MC3D_VARIANT_VOXEL_STEPS) | (ngeoms == 1 ? MC3D_VARIANT_ONE_GEOM : 0);
+    for (const GeomDev &g : gh) p->variant |= photon_variant_wide(g.nx, g.ny, g.nz);
     if (p->math == MC3D_MATH_EXACT) {
         /* division by reciprocal: a step's quotients and their residuals stay normal when
          * the divisors are within [2^-60, 2^60]; a tissue without mu_t is never divided by */

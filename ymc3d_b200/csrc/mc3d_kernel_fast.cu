@@ -10,19 +10,19 @@ namespace mc3d {
 
 /* What bounds them: instruction issue while streams last (80 % of slots; 188
  * thread-instructions a merged step, 283 at first), the fixed latencies of a lone photon's
- * step at a launch's end (0.30 us, 0.62 at first).  1e7 layered photons 221.7 -> 163.4 ms,
- * 1e4 in a pencil beam 11.3 -> 5.4 ms, one step per face (1e6) 180 -> 101 ms.
+ * step at a launch's end (0.30 us, 0.62 at first).  1e7 layered photons 221.7 -> 161.2 ms,
+ * 1e4 in a pencil beam 11.3 -> 5.2 ms, one step per face (1e6) 180 -> 97 ms.
  *
  * 96 registers: 20 warps an SM in blocks of 128 threads, and no spills with one geometry.
- * 80 registers (24 warps) spill 224 bytes: 2.7 % faster on 1e7 layered photons (163.9
- * against 168.3 ms), 5 % slower on twelve mixed geometries and on the grid beyond L2, and a
- * photon's own steps come slower the more warps share an SM (2e5 skin-model photons 4.59
- * against 3.97 ms).  104 registers (16 warps) hide less: 7 % slower on 1e7.
+ * 80 registers (24 warps) spill 160 bytes: 1 % faster on 1e7 and 4e7 layered photons, 1 %
+ * slower on 1e6, per face and on twelve mixed geometries.  64 (32 warps) take 10 % longer on
+ * 1e7, 104 (16 warps) 7 %.
  *
- * Eight instantiations: merged steps (box DDA over uniform cubes) or one step
+ * Thirteen instantiations: merged steps (box DDA over uniform cubes) or one step
  * per voxel face; with or without the absorption map; several geometries (their
  * descriptors in shared memory) or one (its descriptor read from the kernel
- * parameters, which keeps it out of the registers). */
+ * parameters, which keeps it out of the registers); and five of them again for grids
+ * with very long axes. */
 
 /* merged steps */
 __global__ void __maxnreg__(96) photon_kernel_fast(const __grid_constant__ KernelParams P)
@@ -74,11 +74,48 @@ __global__ void __maxnreg__(96)
     photon_kernel_body<MathFast, true, false, true>(P);
 }
 
+/* grids with very long axes */
+__global__ void __maxnreg__(96) photon_kernel_fast_wide(const __grid_constant__ KernelParams P)
+{
+    photon_kernel_body<MathFastWide, false, true>(P);
+}
+
+__global__ void __maxnreg__(96)
+    photon_kernel_fast_wide_amap(const __grid_constant__ KernelParams P)
+{
+    photon_kernel_body<MathFastWide, true, true>(P);
+}
+
+__global__ void __maxnreg__(96)
+    photon_kernel_fast_wide_amap_g1(const __grid_constant__ KernelParams P)
+{
+    photon_kernel_body<MathFastWide, true, true, true>(P);
+}
+
+__global__ void __maxnreg__(96)
+    photon_kernel_fast_wide_voxel(const __grid_constant__ KernelParams P)
+{
+    photon_kernel_body<MathFastWide, false, false>(P);
+}
+
+__global__ void __maxnreg__(96)
+    photon_kernel_fast_wide_voxel_amap(const __grid_constant__ KernelParams P)
+{
+    photon_kernel_body<MathFastWide, true, false>(P);
+}
+
 typedef void (*photon_kernel_t)(KernelParams);
 
 static photon_kernel_t pick(bool amap, int variant)
 {
     const bool voxel = (variant & MC3D_VARIANT_VOXEL_STEPS) != 0;
+    if (variant & MC3D_VARIANT_WIDE) {
+        /* rare: one geometry has its own kernel only where it rounds differently (scatter) */
+        if (voxel) return amap ? photon_kernel_fast_wide_voxel_amap : photon_kernel_fast_wide_voxel;
+        if (!amap) return photon_kernel_fast_wide;
+        return variant & MC3D_VARIANT_ONE_GEOM ? photon_kernel_fast_wide_amap_g1
+                                               : photon_kernel_fast_wide_amap;
+    }
     if (variant & MC3D_VARIANT_ONE_GEOM) {
         if (amap) return voxel ? photon_kernel_fast_voxel_amap_g1 : photon_kernel_fast_amap_g1;
         return voxel ? photon_kernel_fast_voxel_g1 : photon_kernel_fast_g1;
@@ -105,7 +142,11 @@ cudaError_t smem_limit_photon_fast(size_t smem)
     const photon_kernel_t all[] = {photon_kernel_fast,          photon_kernel_fast_amap,
                                    photon_kernel_fast_voxel,    photon_kernel_fast_voxel_amap,
                                    photon_kernel_fast_g1,       photon_kernel_fast_amap_g1,
-                                   photon_kernel_fast_voxel_g1, photon_kernel_fast_voxel_amap_g1};
+                                   photon_kernel_fast_voxel_g1, photon_kernel_fast_voxel_amap_g1,
+                                   photon_kernel_fast_wide,     photon_kernel_fast_wide_amap,
+                                   photon_kernel_fast_wide_amap_g1,
+                                   photon_kernel_fast_wide_voxel,
+                                   photon_kernel_fast_wide_voxel_amap};
     for (photon_kernel_t k : all) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);

@@ -17,6 +17,16 @@ namespace mc3d {
 #define MC3D_VARIANT_ONE_GEOM 4
 /* exact math with IEEE divisions by voxel sizes and mu_t (outside [2^-60, 2^60]) */
 #define MC3D_VARIANT_DIVIDE 8
+/* fast math for grids with more than MC3D_NARROW_DIM voxels along an axis: the other
+ * kernels' voxel indices are exact up to 2^22 */
+#define MC3D_VARIANT_WIDE 16
+#define MC3D_NARROW_DIM (1 << 21)
+
+static inline int photon_variant_wide(int nx, int ny, int nz)
+{
+    return nx > MC3D_NARROW_DIM || ny > MC3D_NARROW_DIM || nz > MC3D_NARROW_DIM
+               ? MC3D_VARIANT_WIDE : 0;
+}
 
 /* dynamic shared memory of a photon kernel: the threads' rows, optical tables, geometry
  * descriptors */

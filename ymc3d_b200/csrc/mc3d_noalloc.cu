@@ -72,6 +72,13 @@ __global__ void __maxnreg__(96)
     photon_kernel_body<MathFast, false, false, true>(P);
 }
 
+/* grids with very long axes */
+__global__ void __maxnreg__(96)
+    photon_kernel_noalloc_wide(const __grid_constant__ KernelParams P)
+{
+    photon_kernel_body<MathFastWide, false, false, true>(P);
+}
+
 /* largest tissue index of the device-resident grid, into a scratch word */
 __global__ void noalloc_max_tissue_kernel(const uint8_t *grid, int64_t n, unsigned int *out)
 {
@@ -274,9 +281,11 @@ extern "C" int mc3d_run_noalloc(const mc3d_geom *geom, const mc3d_props *props,
     NA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const int block = 128; /* at most 28 KB of shared memory: no opt-in */
     size_t smem = photon_smem(P.props_entries, 0, block);
-    NA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, photon_kernel_noalloc, block, smem));
+    const auto kernel = photon_variant_wide(gd.nx, gd.ny, gd.nz) ? photon_kernel_noalloc_wide
+                                                                 : photon_kernel_noalloc;
+    NA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, block, smem));
     if (bps <= 0) return nfail(MC3D_ERR_CAPACITY, "kernel does not fit an SM");
-    photon_kernel_noalloc<<<sms * bps, block, smem, s>>>(P);
+    kernel<<<sms * bps, block, smem, s>>>(P);
     NA_TRY(cudaGetLastError());
     return MC3D_OK;
 }
