@@ -1047,8 +1047,10 @@ __device__ __forceinline__ void photon_kernel_body(const KernelParams &P)
 
     int job = -1;
     unsigned long long *amap = nullptr;
-    const typename M::Geom *gp = nullptr;
-    typename M::Row tab = nullptr;
+    /* valid before the first stream too: a lane that gets none still passes run_chunk,
+     * which names its geometry and table */
+    const typename M::Geom *gp = M::geom(P, sh_geom, 0);
+    typename M::Row tab = M::table(P, sh_tab, 0);
     /* the photon's geometry: the launch's only one from the kernel parameters */
     auto geometry = [&]() -> const typename M::Geom & {
         if constexpr (ONE_GEOM) return P.geom0;
