@@ -7,7 +7,8 @@ import numpy as np
 import pytest
 
 import ymc3d_b200 as m
-from helpers import residual
+from helpers import oracle_job, residual
+from ymc3d_b200 import workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -49,3 +50,23 @@ def test_fewer_streams_than_threads(table, math, steps, streams):
                                                      streams=streams)], **kw)[0]
         assert r.totals["photons"] == 3 * streams
         _same(r, alone)
+
+
+# Voxel sizes so small that the residuals of a quotient by them, and then their
+# reciprocals, leave the normal range: the kernels for such sizes divide along every axis.
+@pytest.mark.parametrize("voxel,optical", [(-112, -112), (-126, -118), (-130, -118)])
+@pytest.mark.parametrize("absorption", [False, True])
+def test_exact_divides_by_tiny_voxels(table, voxel, optical, absorption):
+    g = workloads.layered_vessel_geometry(31, 28, 17, 0.11)
+    g = m.Geometry(g.tissue, *(d * 2.0 ** voxel for d in (0.11, 0.13, 0.07)))
+    p = m.OpticalProps.from_tissues([(a / 2.0 ** optical, s / 2.0 ** optical, gg, n)
+                                     for a, s, gg, n in workloads.LAYER_ROWS])
+    job = m.Job(0, 0, 300, 271828, "uniform")
+    r = m.run([g], [p], [job], table=table, math="exact", photon_log=True, max_steps=5_000,
+              absorption_map=absorption)[0]
+    o = oracle_job(g, p, job, table, photon_log=True, max_steps=5_000,
+                   absorption_map=absorption)
+    assert np.array_equal(_log(r), o["photon_log"].view(np.uint8).reshape(300, -1))
+    assert r.totals == o["totals"] and np.array_equal(r.drs, o["drs"])
+    if absorption:
+        assert np.array_equal(r.absorption, o["absorption"])

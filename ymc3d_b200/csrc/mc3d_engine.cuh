@@ -256,6 +256,7 @@ struct MathExact : FloatTable {
 /* The same with IEEE divisions, for voxel sizes and coefficients whose reciprocals, or
  * the residuals of the quotients, leave FP32's normal range. */
 struct MathExactWide : MathExact {
+    using Pairs = PairwiseOps<MathExactWide, float>; /* x and y divide too */
     static __device__ __forceinline__ float div_r(float a, float b, float) { return a / b; }
     static __device__ __forceinline__ float advance(float x, float us, bool hit, float t, float mu_t,
                                                     float)
