@@ -70,3 +70,22 @@ def test_exact_divides_by_tiny_voxels(table, voxel, optical, absorption):
     assert r.totals == o["totals"] and np.array_equal(r.drs, o["drs"])
     if absorption:
         assert np.array_equal(r.absorption, o["absorption"])
+
+
+# With g = 0 the scattering cosine is 0/0, so a photon has no position after its first
+# scattering.  Until the quickfix removes it, its absorbed weight goes to the voxel its
+# tissue is looked up in: the first one in FP32, the last one in FP64.
+@pytest.mark.parametrize("math,steps", MODES)
+def test_absorption_without_a_position(table, math, steps):
+    t = np.ones((9, 7, 11), np.uint8)
+    p = m.OpticalProps.from_tissues([(1.0, 5.0, 0.0, 1.4)])
+    r = m.run([m.Geometry(t, 0.1, 0.1, 0.1)], [p], [m.Job(0, 0, 500, 77, "pencil")],
+              table=table, math=math, steps=steps, absorption_map=True)[0]
+    a = r.absorption.copy()
+    assert int(a.sum()) == r.totals["absorbed"] and r.totals["quickfix"] > 0
+    corners = [(0, 0, 0), (8, 6, 10)]
+    lost, none = corners[::-1] if math == "f64" else corners
+    assert a[lost] > 0 and a[none] == 0
+    a[lost] = 0
+    a[:, 3, 5] = 0  # the beam's column
+    assert not a.any()

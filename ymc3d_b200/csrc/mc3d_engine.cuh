@@ -666,10 +666,11 @@ static __device__ __forceinline__ bool photon_step(const typename M::Geom &g, ty
         /* absorption map, the reference's disabled tally (src/mc3d_gpu.cu:265-272):
          * the current voxel clamped into the grid, fixed-point weight removed.  A
          * merged step can end its flight several voxels from where it started, so
-         * there the voxel of the interaction point is used. */
-        const int ai = min(max((int)(JUMP ? nexti : p.i), 0), g.nx - 1);
-        const int aj = min(max((int)(JUMP ? nextj : p.j), 0), g.ny - 1);
-        const int ak = min(max((int)(JUMP ? nextk : p.k), 0), g.nz - 1);
+         * there the voxel of the interaction point is used.  A photon without a
+         * position (NaN, of a tissue with g = 0) tallies where its cell is looked up. */
+        const int ai = M::cell(JUMP ? nexti : p.i, g.last_x);
+        const int aj = M::cell(JUMP ? nextj : p.j, g.last_y);
+        const int ak = M::cell(JUMP ? nextk : p.k, g.nz - 1);
         const uint64_t dq = M::qw(p.W) - M::qw(W);
         if (dq) atomicAdd(amap + ((int64_t)ak * g.ny + aj) * g.nx + ai, (unsigned long long)dq);
     }
