@@ -89,3 +89,22 @@ def test_absorption_without_a_position(table, math, steps):
     a[lost] = 0
     a[:, 3, 5] = 0  # the beam's column
     assert not a.any()
+
+
+# Fast math flushes denormals, so a tissue whose mu_t is one stops a photon as air does;
+# FP64 and exact math do not.
+@pytest.mark.parametrize("steps", ["merged", "voxel"])
+@pytest.mark.parametrize("mua,mus", [(1e-42, 0.0), (0.0, 1e-40), (3e-39, 4e-39)])
+@pytest.mark.parametrize("n", [1.4, 1.33])
+def test_denormal_mu_t_is_zero(table, steps, mua, mus, n):
+    t = np.ones((12, 10, 14), np.uint8)
+    t[7:] = 2
+    t[:4, 2:5, 3:6] = 2
+    g = m.Geometry(t, 0.1, 0.1, 0.1)
+    runs = []
+    for a, s in ((0.0, 0.0), (mua, mus)):
+        p = m.OpticalProps.from_tissues([(0.2, 8.0, 0.8, 1.4), (a, s, 0.8, n)])
+        runs.append(m.run([g], [p], [m.Job(0, 0, 3000, 5, "uniform")], table=table, steps=steps,
+                          photon_log=True, max_steps=20_000)[0])
+    assert runs[0].totals["t_in"] > 0 and runs[0].totals["capped"] == 0
+    _same(*runs)
