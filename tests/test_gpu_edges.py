@@ -108,3 +108,18 @@ def test_denormal_mu_t_is_zero(table, steps, mua, mus, n):
                           photon_log=True, max_steps=20_000)[0])
     assert runs[0].totals["t_in"] > 0 and runs[0].totals["capped"] == 0
     _same(*runs)
+
+
+@pytest.mark.parametrize("mua,mus", [(-50.0, 60.0), (-120.0, 150.0)])
+def test_exact_follows_a_gain_medium(table, mua, mus):
+    """A weight that grows beyond FP32's range: still the CPU transcription's photons."""
+    t = np.ones((12, 10, 14), np.uint8)
+    t[6:] = 2
+    g = m.Geometry(t, 0.1, 0.1, 0.1)
+    p = m.OpticalProps.from_tissues([(mua, mus, 0.8, 1.4), (0.5, 5.0, 0.6, 1.33)])
+    job = m.Job(0, 0, 300, 99, "uniform")
+    r = m.run([g], [p], [job], table=table, math="exact", photon_log=True, max_steps=3_000)[0]
+    o = oracle_job(g, p, job, table, photon_log=True, max_steps=3_000)
+    assert np.isnan(o["photon_log"]["W"]).any()
+    for k in r.photon_log.dtype.names:
+        assert np.array_equal(r.photon_log[k], o["photon_log"][k], equal_nan=True), k

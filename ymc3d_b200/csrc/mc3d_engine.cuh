@@ -668,8 +668,16 @@ static __device__ __forceinline__ bool photon_step(const typename M::Geom &g, ty
     rx = mc3d_mwc_next(rx, ra);
     uint32_t e_s = (uint32_t)rx;
 
-    /* absorption, src/mc3d_gpu.cu:262-263 */
-    R W = p.W - (hit ? (R)0 : M::mul(M::albedo_c(tt), p.W));
+    /* Absorption, src/mc3d_gpu.cu:262-263.  Fast math selects; the others multiply by 0 or
+     * 1 as the reference does, which makes an infinite weight (a medium with gain) NaN at
+     * the next face. */
+    R W;
+    if (M::kFast) {
+        W = p.W - (hit ? (R)0 : M::mul(M::albedo_c(tt), p.W));
+    } else {
+        const R dW = mu_t > 0 ? M::mul(M::albedo_c(tt), p.W) : (R)0;
+        W = p.W - M::mul(dW, hit ? (R)0 : (R)1);
+    }
     if (AMAP && !hit && mu_t > 0) {
         /* absorption map, the reference's disabled tally (src/mc3d_gpu.cu:265-272):
          * the current voxel clamped into the grid, fixed-point weight removed.  A
