@@ -611,6 +611,7 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
         for (int t = 0; t < props[i].num_tissue_types; t++) {
             float mua = props[i].mua[t], mus = props[i].mus[t], g = props[i].g[t];
             volatile float mut = mua + mus;
+            if (p->math == MC3D_MATH_FAST) mut = flushed_mu_t(mut);
             volatile float frac = mut > 0 ? mua / mut : 0.0f, rmut = 1.0f / mut, g2 = g * g, twog = 2 * g;
             volatile float inv2g = 1.0f / twog;
             float4 *e = &tab[props_offset[i] + 3 * t];

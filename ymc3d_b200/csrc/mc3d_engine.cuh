@@ -192,35 +192,28 @@ struct FloatTable {
     static __device__ __forceinline__ float zero_threshold() { return (float)(1 - 0.99999); }
     /* Whether a step needs the work that few do (photon_step).  One chain of compares,
      * each taking the result so far: written in C the terms are combined by predicate
-     * instructions of their own (8.6 of the step's 192, 5.2 of 188 this way).  FTZ is
-     * ".ftz" for fast math, whose mu_t below the normal range is 0 here as in the rest of
-     * the step; the other values are results, already flushed, or bounds. */
-#define MC3D_RARE_CHAIN(FTZ)                                                                   \
-    asm("{\n\t.reg .pred p;\n\t"                                                              \
-        "setp.ne.u32 p, %1, 0;\n\t"                                                            \
-        "setp.leu.or.f32 p, %2, %3, p;\n\t"                                                    \
-        "setp.eq.or" FTZ ".f32 p, %4, 0f00000000, p;\n\t"                                      \
-        "setp.gtu.or.f32 p, %5, %6, p;\n\t"                                                    \
-        "setp.lt.or.f32 p, %7, %8, p;\n\t"                                                     \
-        "setp.leu.or.f32 p, %9, 0f00000000, p;\n\t"                                            \
-        "setp.geu.or.f32 p, %9, %10, p;\n\t"                                                   \
-        "setp.leu.or.f32 p, %11, 0f00000000, p;\n\t"                                           \
-        "setp.geu.or.f32 p, %11, %12, p;\n\t"                                                  \
-        "selp.u32 %0, 1, 0, p;\n\t}"                                                           \
-        : "=r"(any)                                                                            \
-        : "r"(changed), "f"(W), "f"(0x1.a36e2ep-14f), "f"(mu_t), "f"(fabsf(uz)),                \
-          "f"(0x1.fffeb0p-1f), "f"(least_u), "f"(zero_threshold()), "f"(x), "f"(Lx), "f"(y),    \
-          "f"(Ly))
-    template <bool FAST>
+     * instructions of their own (8.6 of the step's 192, 5.2 of 188 this way). */
     static __device__ __forceinline__ bool rare(uint32_t changed, float W, float mu_t, float uz,
                                                 float least_u, float x, float Lx, float y, float Ly)
     {
         uint32_t any;
-        if constexpr (FAST) MC3D_RARE_CHAIN(".ftz");
-        else MC3D_RARE_CHAIN("");
+        asm("{\n\t.reg .pred p;\n\t"
+            "setp.ne.u32 p, %1, 0;\n\t"
+            "setp.leu.or.f32 p, %2, %3, p;\n\t"
+            "setp.eq.or.f32 p, %4, 0f00000000, p;\n\t"
+            "setp.gtu.or.f32 p, %5, %6, p;\n\t"
+            "setp.lt.or.f32 p, %7, %8, p;\n\t"
+            "setp.leu.or.f32 p, %9, 0f00000000, p;\n\t"
+            "setp.geu.or.f32 p, %9, %10, p;\n\t"
+            "setp.leu.or.f32 p, %11, 0f00000000, p;\n\t"
+            "setp.geu.or.f32 p, %11, %12, p;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(any)
+            : "r"(changed), "f"(W), "f"(0x1.a36e2ep-14f), "f"(mu_t), "f"(fabsf(uz)),
+              "f"(0x1.fffeb0p-1f), "f"(least_u), "f"(zero_threshold()), "f"(x), "f"(Lx), "f"(y),
+              "f"(Ly));
         return any != 0;
     }
-#undef MC3D_RARE_CHAIN
     /* fixed-point weight, 2^-32 resolution */
     static __device__ __forceinline__ uint64_t qw(float w) { return __float2ull_rn(w * 4294967296.0f); }
 };
@@ -403,7 +396,6 @@ struct MathF64 {
     static __device__ __forceinline__ bool uz_within(double u) { return u <= 0.99999; }
     static __device__ __forceinline__ double roulette_survivor(double w) { return w / 0.1; }
     static __device__ __forceinline__ double zero_threshold() { return 1 - 0.99999; }
-    template <bool FAST>
     static __device__ __forceinline__ bool rare(uint32_t changed, double W, double mu_t, double uz,
                                                 double least_u, double x, double Lx, double y,
                                                 double Ly)
@@ -719,7 +711,7 @@ static __device__ __forceinline__ bool photon_step(const typename M::Geom &g, ty
     const bool steep = !M::uz_within(M::fabs(p.uz));
     const uint32_t changed = (uint32_t)(next_tissue ^ p.tissue) & 0xffu;
     const R least_u = M::fmin(M::fabs(nux), M::fmin(M::fabs(nuy), M::fabs(nuz)));
-    if (M::template rare<M::kFast>(changed, W, mu_t, p.uz, least_u, newx, g.Lx, newy, g.Ly)) {
+    if (M::rare(changed, W, mu_t, p.uz, least_u, newx, g.Lx, newy, g.Ly)) {
         bool refl = false;
         bool again = steep && !hit;   /* the scattering anew */
         bool redo = steep | (least_u < zero_thresh); /* the normalisation anew */

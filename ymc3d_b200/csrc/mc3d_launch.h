@@ -6,6 +6,8 @@
 #ifndef MC3D_LAUNCH_H
 #define MC3D_LAUNCH_H
 
+#include <float.h>
+#include <math.h>
 #include <cuda_runtime.h>
 #include "mc3d_device_types.h"
 
@@ -27,6 +29,9 @@ static inline int photon_variant_wide(int nx, int ny, int nz)
     return nx > MC3D_NARROW_DIM || ny > MC3D_NARROW_DIM || nz > MC3D_NARROW_DIM
                ? MC3D_VARIANT_WIDE : 0;
 }
+
+/* mu_t as fast math's kernels, which flush denormals, have it in every expression */
+static inline float flushed_mu_t(float mut) { return fabsf(mut) < FLT_MIN ? 0.0f : mut; }
 
 /* dynamic shared memory of a photon kernel: the threads' rows, optical tables, geometry
  * descriptors */

@@ -184,7 +184,7 @@ extern "C" int mc3d_run_noalloc(const mc3d_geom *geom, const mc3d_props *props,
     float4 tab[MC3D_TAB_STRIDE * MC3D_NOALLOC_MAX_TISSUES];
     for (int t = 0; t < nt; t++) {
         float mua = props->mua[t], mus = props->mus[t], g = props->g[t];
-        volatile float mut = mua + mus;
+        volatile float mut = flushed_mu_t(mua + mus);
         volatile float frac = mut > 0 ? mua / mut : 0.0f, rmut = 1.0f / mut, g2 = g * g, twog = 2 * g;
         volatile float inv2g = 1.0f / twog;
         tab[3 * t + 0] = make_float4(mua, mus, g, props->n[t]);
