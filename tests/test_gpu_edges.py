@@ -3,10 +3,14 @@ coefficients below the normal range, photons without a position, memory and tabl
 their limits."""
 from __future__ import annotations
 
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 import ymc3d_b200 as m
+from conftest import ROOT
 from helpers import oracle_job, residual
 from ymc3d_b200 import workloads
 
@@ -124,3 +128,63 @@ def test_exact_follows_a_gain_medium(table, mua, mus):
     assert np.isnan(o["photon_log"]["W"]).any()
     for k in r.photon_log.dtype.names:
         assert np.array_equal(r.photon_log[k], o["photon_log"][k], equal_nan=True), k
+
+
+def _in_fresh_process(code):
+    """the process's last line of output; its library starts with an empty memory pool"""
+    run = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True,
+                         timeout=300)
+    assert run.returncode == 0, run.stdout + run.stderr
+    return run.stdout.splitlines()[-1]
+
+
+_PLAN = """
+import sys
+sys.path.insert(0, ".")
+import numpy as np, torch
+import ymc3d_b200 as m
+MiB = 1 << 20
+free = lambda: torch.cuda.mem_get_info()[0]
+dev = torch.device("cuda", 0)
+torch.zeros(1, device=dev)
+def fill(leave):
+    torch.cuda.synchronize()
+    return torch.empty(free() - leave, dtype=torch.uint8, device=dev)
+"""
+
+
+def test_optional_states_leave_room_for_the_rest():
+    """A plan keeps its streams' states (8 bytes each, 512 MiB here) only beside what it
+    cannot do without: an absorption map (512 MiB) that fits without them still fits, and
+    the photons are the same either way."""
+    out = _in_fresh_process(_PLAN + """
+g = m.Geometry(np.ones((256, 512, 512), np.uint8), 0.05, 0.05, 0.05)
+p = m.OpticalProps.from_tissues([(50.0, 5.0, 0.5, 1.4)])
+job = m.Job(0, 0, 1 << 26, 7, "uniform")
+m.run([m.Geometry(np.ones((2, 2, 2), np.uint8), 1, 1, 1)], [p], [m.Job(0, 0, 10, 7)])
+hold = fill(64 * MiB + 2 * 512 * 512 * 319 + 512 * MiB + 200 * MiB)
+a = m.run([g], [p], [job], absorption_map=True)[0]
+del hold
+torch.cuda.empty_cache()
+b = m.run([g], [p], [job], absorption_map=True)[0]
+assert a.totals == b.totals and a.totals["photons"] == 1 << 26
+assert np.array_equal(a.drs, b.drs) and np.array_equal(a.absorption, b.absorption)
+print("same")
+""")
+    assert out == "same"
+
+
+def test_states_are_given_back_after_a_rejection():
+    """A rejected seeding attempt makes the kept states useless: their memory (128 MiB) serves
+    the next plan."""
+    out = _in_fresh_process(_PLAN + """
+table = m.default_table().copy()
+table[1 + 12345] = 3
+g = m.Geometry(np.ones((4, 4, 4), np.uint8), 0.1, 0.1, 0.1)
+p = m.OpticalProps.from_tissues([(5.0, 5.0, 0.5, 1.4)])
+plans = [m.Plan([g], [p], [m.Job(0, 0, 1 << 24, 7, "uniform")], table)]
+before = free()
+plans.append(m.Plan([g], [p], [m.Job(0, 0, 1 << 24, 8, "uniform")], table))
+print((before - free()) // MiB)
+""")
+    assert int(out) < 64
