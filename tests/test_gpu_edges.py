@@ -8,6 +8,7 @@ import sys
 
 import numpy as np
 import pytest
+import torch
 
 import ymc3d_b200 as m
 from conftest import ROOT
@@ -188,3 +189,28 @@ plans.append(m.Plan([g], [p], [m.Job(0, 0, 1 << 24, 8, "uniform")], table))
 print((before - free()) // MiB)
 """)
     assert int(out) < 64
+
+
+def _many_sets(n):
+    """n optical sets of five tissues, 240 bytes each in a block's shared memory"""
+    return [m.OpticalProps.from_tissues([(a * (0.5 + k / n), s, g, i)
+                                         for a, s, g, i in workloads.LAYER_ROWS])
+            for k in range(n)]
+
+
+# An SM has 228 KB for each block's tables, 136 bytes a thread and 1 KB a block, and registers
+# for 20 warps in FP32: the most warps that fit in blocks of 128 to 256 threads.
+@pytest.mark.parametrize("math", ["fast", "exact"])
+@pytest.mark.parametrize("sets,warps", [(20, 20), (120, 20), (180, 18), (340, 14), (360, 12)])
+def test_large_tables_keep_warps(table, math, sets, warps):
+    g = m.Geometry(_blocks(7, (4, 5, 4), 4), 0.05, 0.05, 0.05)
+    props = _many_sets(sets)
+    jobs = [m.Job(0, k, 40, 100 + k, "uniform") for k in range(sets)]
+    plan = m.Plan([g], props, jobs, table=table, math=math)
+    block, grid, smem = plan.shape()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert grid % sms == 0 and block * grid // sms == 32 * warps
+    plan.execute()
+    for a, b in zip(plan.read(), m.run([g], props, jobs, table=table, math=math, block=64)):
+        _same(a, b)
+    plan.close()

@@ -716,12 +716,14 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
             if (tab[i + 1].x != 0) check(tab[i + 1].x);
         if (wide) p->variant |= MC3D_VARIANT_DIVIDE;
     }
-    /* 128 threads, of whose registers an SM holds 20 warps of the fast kernel (16 in
-     * blocks of 256), unless the optical tables, of which each block has a copy, leave
-     * room for more threads in larger blocks */
+    /* 128 threads, of whose registers an SM holds 20 warps of the fast kernel, unless the
+     * optical tables, of which each block has a copy, leave room for more threads in fewer
+     * and larger blocks.  2e6 photons in blocks of tissue of 4^3 voxels, tables of 42 KB:
+     * 13.6 ms with 3 blocks of 192, 14.2 with 2 of 256; of 80 KB: 15.6 ms with 2 of 224, 22.9
+     * with 2 of 128 or 1 of 256. */
     int bps = 0;
-    for (int block : {opt.block ? (int)opt.block : 128, opt.block ? 0 : 256}) {
-        if (block == 0) continue;
+    for (int block = opt.block ? opt.block : 128; block <= (opt.block ? opt.block : 256);
+         block += 32) {
         int n = 0;
         const size_t smem = photon_smem(entries, ngeoms, block);
         PLAN_TRY(p->math == MC3D_MATH_FAST ? occupancy_photon_fast(block, smem, &n, p->variant)
