@@ -214,3 +214,23 @@ def test_large_tables_keep_warps(table, math, sets, warps):
     for a, b in zip(plan.read(), m.run([g], props, jobs, table=table, math=math, block=64)):
         _same(a, b)
     plan.close()
+
+
+def test_fp64_tables_take_no_shared_memory(table):
+    """FP64 stepping reads its tables from global memory: their size leaves its 16 warps an SM
+    and the L1 cache alone."""
+    g = m.Geometry(_blocks(7, (4, 5, 4), 4), 0.05, 0.05, 0.05)
+    shapes = []
+    for sets in (1, 340, 800):
+        props = _many_sets(sets)
+        jobs = [m.Job(0, k, 20, 100 + k, "uniform") for k in range(sets)]
+        plan = m.Plan([g], props, jobs, table=table, math="f64")
+        shapes.append(plan.shape())
+        plan.execute()
+        last = plan.read()[-1]
+        plan.close()
+        _same(last, m.run([g], props[-1:], [m.Job(0, 0, 20, 99 + sets, "uniform")], table=table,
+                          math="f64")[0])
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert shapes[0] == shapes[1] == shapes[2]
+    assert shapes[0][0] * shapes[0][1] // sms == 512

@@ -681,6 +681,9 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
     PLAN_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, p->device));
     PLAN_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
                                     p->device));
+    /* FP64 stepping reads tables and geometries through L1, which shares its memory */
+    const int shared_entries = p->math == MC3D_MATH_F64 ? 0 : entries;
+    const int shared_geoms = p->math == MC3D_MATH_F64 ? 0 : ngeoms;
     /* The kernels always opt in to the device's whole per-block limit of shared
      * memory: the attribute is per function, and a lower value would break a live
      * plan that needs more. */
@@ -690,7 +693,7 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
                  : p->math == MC3D_MATH_EXACT ? attributes_photon_exact(&fa)
                                               : attributes_photon_f64(&fa));
         const size_t max_dyn = (size_t)smem_optin - fa.sharedSizeBytes;
-        p->smem = photon_smem(entries, ngeoms, opt.block ? opt.block : 128);
+        p->smem = photon_smem(shared_entries, shared_geoms, opt.block ? opt.block : 128);
         if (p->smem > max_dyn) {
             plan_free(p);
             return fail(MC3D_ERR_CAPACITY, "optical tables and geometry descriptors need %zu B "
@@ -725,7 +728,7 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
     for (int block = opt.block ? opt.block : 128; block <= (opt.block ? opt.block : 256);
          block += 32) {
         int n = 0;
-        const size_t smem = photon_smem(entries, ngeoms, block);
+        const size_t smem = photon_smem(shared_entries, shared_geoms, block);
         PLAN_TRY(p->math == MC3D_MATH_FAST ? occupancy_photon_fast(block, smem, &n, p->variant)
                  : p->math == MC3D_MATH_EXACT ? occupancy_photon_exact(block, smem, &n, p->variant)
                                               : occupancy_photon_f64(block, smem, &n, p->variant));
