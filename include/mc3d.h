@@ -145,8 +145,9 @@ typedef struct {
 typedef struct {
     int32_t device;         /* CUDA device ordinal */
     int32_t math;           /* enum mc3d_math */
-    int32_t block;          /* threads per block, 0 = tuned */
-    int32_t blocks_per_sm;  /* 0 = as many as fit */
+    int32_t block;          /* threads per block, a multiple of 32 up to 256; 0 = the size
+                               from 128 up that gives an SM the most threads */
+    int32_t blocks_per_sm;  /* at most so many blocks; 0 = as many as fit */
     int32_t absorption_map; /* 1: tally absorbed weight per voxel (sum over voxels = absorbed) */
     int32_t use_graph;      /* 1: a plan's first execute captures the tally clear and the
                                launch into a CUDA graph, later executes replay it */

@@ -234,3 +234,24 @@ def test_fp64_tables_take_no_shared_memory(table):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert shapes[0] == shapes[1] == shapes[2]
     assert shapes[0][0] * shapes[0][1] // sms == 512
+
+
+# Without a block size, a limit on the blocks leaves an SM as many threads as it can: blocks
+# of 256 for one or two (16 warps is what fits of them), then what gives more.
+@pytest.mark.parametrize("math", ["fast", "exact", "f64"])
+@pytest.mark.parametrize("limit,warps", [(1, 8), (2, 16), (3, 18), (4, 20), (5, 20), (9, 20)])
+def test_block_limit_counts_the_largest_blocks(table, math, limit, warps):
+    g = m.Geometry(np.ones((8, 8, 8), np.uint8), 0.1, 0.1, 0.1)
+    p = m.OpticalProps.from_tissues([(1.0, 10.0, 0.9, 1.4)])
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    job = m.Job(0, 0, 500, 3, "uniform")
+    plan = m.Plan([g], [p], [job], table=table, math=math, blocks_per_sm=limit)
+    block, grid, _ = plan.shape()
+    assert grid // sms <= limit
+    assert block * grid // sms == 32 * min(warps, 16 if math == "f64" else 20)
+    plan.execute()
+    _same(plan.read()[0], m.run([g], [p], [job], table=table, math=math)[0])
+    plan.close()
+    plan = m.Plan([g], [p], [job], table=table, math=math, block=64, blocks_per_sm=limit)
+    assert plan.shape()[:2] == (64, sms * min(limit, 8 if math == "f64" else 9))
+    plan.close()

@@ -723,7 +723,8 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
      * optical tables, of which each block has a copy, leave room for more threads in fewer
      * and larger blocks.  2e6 photons in blocks of tissue of 4^3 voxels, tables of 42 KB:
      * 13.6 ms with 3 blocks of 192, 14.2 with 2 of 256; of 80 KB: 15.6 ms with 2 of 224, 22.9
-     * with 2 of 128 or 1 of 256. */
+     * with 2 of 128 or 1 of 256.  A caller's limit on the blocks
+     * counts in: blocks of 256 threads for one or two, of 192 for three. */
     int bps = 0;
     for (int block = opt.block ? opt.block : 128; block <= (opt.block ? opt.block : 256);
          block += 32) {
@@ -732,6 +733,7 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
         PLAN_TRY(p->math == MC3D_MATH_FAST ? occupancy_photon_fast(block, smem, &n, p->variant)
                  : p->math == MC3D_MATH_EXACT ? occupancy_photon_exact(block, smem, &n, p->variant)
                                               : occupancy_photon_f64(block, smem, &n, p->variant));
+        if (opt.blocks_per_sm > 0) n = std::min(n, (int)opt.blocks_per_sm);
         if (n * block > bps * p->block || p->block == 0) {
             p->block = block;
             p->smem = smem;
@@ -742,7 +744,6 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
         plan_free(p);
         return fail(MC3D_ERR_CAPACITY, "kernel does not fit an SM with block %d", opt.block);
     }
-    if (opt.blocks_per_sm > 0) bps = std::min(bps, (int)opt.blocks_per_sm);
     p->grid = num_sms * bps;
 
     /* ---- the seeding scan for rejected attempts */
