@@ -4,17 +4,18 @@ Tallies do not depend on the launch shape (streams, not threads, own the random
 numbers), so the shape is a pure speed choice.  The tuner runs a sample of the
 real jobs -- the first streams of each -- under each candidate (threads per
 block, blocks per SM), times it with CUDA events and keeps the fastest.  Choices
-are cached per (device name, workload signature) in memory and in
-_data/tuning.json next to the library.
+are cached per (device name, workload signature, build of the library, candidates)
+in memory and in _data/tuning.json next to the library.
 """
 from __future__ import annotations
 
+import functools
 import hashlib
 import json
 import os
 import time
 
-from . import HERE, Job, Plan, default_table
+from . import HERE, LIB_PATH, Job, Plan, default_table
 
 # (threads per block, blocks per SM; 0 = as many as fit).  The fast and exact kernels are
 # built for 96 registers: 5 blocks of 128 threads fill an SM (20 warps), 2 of 256 hold 16
@@ -59,6 +60,27 @@ def signature(geoms, props, jobs, math: str, steps: str = "merged") -> str:
     return h.hexdigest()[:16]
 
 
+@functools.cache
+def _build_id(path=LIB_PATH) -> str:
+    """Of the library: another build's kernels have other registers, and other best shapes."""
+    return hashlib.sha1(path.read_bytes()).hexdigest()[:16]
+
+
+def cache_key(device_name: str, sig: str, candidates=CANDIDATES) -> str:
+    shapes = hashlib.sha1(repr(tuple(map(tuple, candidates))).encode()).hexdigest()[:8]
+    return f"{device_name}|{sig}|{_build_id()}|{shapes}"
+
+
+def choose(results: list[dict]) -> dict:
+    """The fastest shape.  The sample's tail is a larger share of it than the launch's and
+    favours fewer warps, so a shape that holds fewer threads than the first has to win by
+    more than 2 %.  (Per-face steps, 1e7 photons: 681 ms with 20 warps an SM and 711 with
+    16, which won the sample by 0.2 %.)"""
+    threads = results[0]["block"] * results[0]["grid"]
+    return min(results, key=lambda r: r["ms"] * (1.02 if r["block"] * r["grid"] < threads
+                                                 else 1.0))
+
+
 def _sample_jobs(jobs, streams_per_job: int):
     out = []
     for j in jobs:
@@ -75,7 +97,7 @@ def tune(geoms, props, jobs, table=None, math: str = "fast", device: int = 0,
     import torch
 
     dev_name = torch.cuda.get_device_name(device)
-    key = f"{dev_name}|{signature(geoms, props, jobs, math, steps)}"
+    key = cache_key(dev_name, signature(geoms, props, jobs, math, steps), candidates)
     cache = _load()
     if use_cache and key in cache:
         return cache[key]
@@ -111,10 +133,7 @@ def tune(geoms, props, jobs, table=None, math: str = "fast", device: int = 0,
         plan.close()
     if not results:
         raise RuntimeError("no launch shape could be planned")
-    # The sample's tail is a larger share of it than the launch's and favours fewer warps:
-    # a shape that holds fewer than the first has to win by more than 2 %.  (Per-face steps,
-    # 1e7 photons: 681 ms with 20 warps an SM and 711 with 16, which won the sample by 0.2 %.)
-    best = min(results, key=lambda r: r["ms"] * (1.0 if r is results[0] else 1.02))
+    best = choose(results)
     choice = {"block": best["block"], "blocks_per_sm": best["blocks_per_sm"], "ms": best["ms"],
               "table": results, "when": time.strftime("%Y-%m-%dT%H:%M:%S")}
     cache[key] = choice
