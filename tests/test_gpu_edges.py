@@ -13,7 +13,7 @@ import torch
 import ymc3d_b200 as m
 from conftest import ROOT
 from helpers import oracle_job, residual
-from ymc3d_b200 import workloads
+from ymc3d_b200 import autotune, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -255,3 +255,15 @@ def test_block_limit_counts_the_largest_blocks(table, math, limit, warps):
     plan = m.Plan([g], [p], [job], table=table, math=math, block=64, blocks_per_sm=limit)
     assert plan.shape()[:2] == (64, sms * min(limit, 8 if math == "f64" else 9))
     plan.close()
+
+
+def test_autotuner_starts_from_the_plans_shape(table):
+    """42 KB of tables: a plan takes 3 blocks of 192, which the tuner times first"""
+    g = m.Geometry(_blocks(7, (4, 5, 4), 4), 0.05, 0.05, 0.05)
+    props = _many_sets(180)
+    jobs = [m.Job(0, k, 40, 100 + k, "uniform") for k in range(180)]
+    plan = m.Plan([g], props, jobs, table=table)
+    block, grid, _ = plan.shape()
+    plan.close()
+    first = autotune.tune([g], props, jobs, table=table, use_cache=False)["table"][0]
+    assert (first["block"], first["grid"]) == (block, grid) and block == 192

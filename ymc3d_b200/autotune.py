@@ -17,11 +17,12 @@ import time
 
 from . import HERE, LIB_PATH, Job, Plan, default_table
 
-# (threads per block, blocks per SM; 0 = as many as fit).  The fast and exact kernels are
-# built for 96 registers: 5 blocks of 128 threads fill an SM (20 warps), 2 of 256 hold 16
-# warps.  Fewer warps hide less latency but let each photon step sooner, which shortens
-# the end of a launch of few photons per thread.
-CANDIDATES = ((128, 0), (128, 4), (128, 3), (256, 0))
+# (threads per block, blocks per SM); 0 threads = the plan's own choice, 0 blocks = as many
+# as fit.  The fast and exact kernels are built for 96 registers: a plan takes 5 blocks of
+# 128 threads (20 warps an SM), or larger ones where optical tables fill the shared memory.
+# Fewer warps hide less latency but let each photon step sooner, which shortens the end of
+# a launch of few photons per thread.
+CANDIDATES = ((0, 0), (128, 4), (128, 3), (256, 0))
 _CACHE_FILE = HERE / "_data" / "tuning.json"
 _cache: dict | None = None
 
@@ -128,8 +129,8 @@ def tune(geoms, props, jobs, table=None, math: str = "fast", device: int = 0,
             e1.record(stream)
             e1.synchronize()
             times.append(e0.elapsed_time(e1))
-        results.append({"block": block, "blocks_per_sm": bps, "ms": min(times),
-                        "grid": plan.shape()[1]})
+        threads, grid, _ = plan.shape()
+        results.append({"block": threads, "blocks_per_sm": bps, "ms": min(times), "grid": grid})
         plan.close()
     if not results:
         raise RuntimeError("no launch shape could be planned")
