@@ -12,7 +12,7 @@ import torch
 
 import ymc3d_b200 as m
 from conftest import ROOT
-from helpers import oracle_job, residual
+from helpers import oracle_job, residual, safe_distance_bruteforce
 from ymc3d_b200 import autotune, workloads
 
 pytestmark = pytest.mark.gpu
@@ -267,3 +267,39 @@ def test_autotuner_starts_from_the_plans_shape(table):
     plan.close()
     first = autotune.tune([g], props, jobs, table=table, use_cache=False)["table"][0]
     assert (first["block"], first["grid"]) == (block, grid) and block == 192
+
+
+@pytest.mark.parametrize("shape", [(5, 7, 1), (5, 1, 7), (9, 6, 2), (9, 2, 6), (4, 5, 3), (1, 2, 1),
+                                   (66, 3, 3)])
+def test_narrow_grids(table, shape):
+    """Grids whose voxels all lie on a lateral face, and the narrowest others: maps by
+    definition, and merged steps as steps at every face (the tissues differ in index)."""
+    t = np.random.default_rng(sum(shape)).integers(1, 4, shape).astype(np.uint8)
+    t[shape[0] // 2:] = 1
+    assert np.array_equal(m.safe_distance(t), safe_distance_bruteforce(t))
+    p = m.OpticalProps.from_tissues([(0.5, 9.0, 0.9, 1.4), (1.0, 5.0, 0.7, 1.33),
+                                     (0.8, 20.0, 0.8, 1.5)])
+    a, b = (m.run([m.Geometry(t, 0.1, 0.12, 0.09)], [p], [m.Job(0, 0, 400, 3, "uniform")],
+                  table=table, photon_log=True, steps=steps)[0] for steps in ("merged", "voxel"))
+    if min(shape[1:]) <= 2:
+        _same(a, b)
+    assert residual(a.totals) == 0
+
+
+def test_narrow_grid_needs_no_padded_maps():
+    """One voxel wide, three tissues of two indices: cells and grid fit where maps of four
+    bytes a voxel would not."""
+    out = _in_fresh_process(_PLAN + """
+n = 16384
+t = np.ones((n - 63, n, 1), np.uint8)
+t[100:200] = 2
+t[200:300] = 3
+g = m.Geometry(t, 0.1, 0.1, 0.1)
+p = m.OpticalProps.from_tissues([(1.0, 9.0, 0.9, 1.4), (1.0, 5.0, 0.7, 1.4), (1.0, 5.0, 0.7, 1.3)])
+m.run([m.Geometry(t[:2, :2], 1, 1, 1)], [p], [m.Job(0, 0, 10, 7)])
+hold = fill(7 * n * n + 200 * MiB)
+plan = m.Plan([g], [p], [m.Job(0, 0, 1000, 7, "uniform")])
+plan.execute()
+print(plan.read()[0].photons)
+""")
+    assert int(out) == 1000

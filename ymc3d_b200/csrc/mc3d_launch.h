@@ -67,7 +67,8 @@ cudaError_t launch_seed_scan(const JobDev *jobs, int njobs, const uint32_t *mult
 cudaError_t launch_seed_dump(const KernelParams &P, int64_t first, int64_t count,
                              uint64_t *x_out, uint32_t *a_out, cudaStream_t stream);
 /* bytes of scratch that the two launches below need for a grid: two maps of whole
- * words a row, three with the distances of the refractive-index classes */
+ * words a row, three with the distances of the refractive-index classes; none for a grid
+ * at most two voxels wide */
 size_t safe_distance_scratch(int nx, int ny, int nz, bool index_map);
 /* safe-distance map of a tissue grid: nx * ny * (nz + MC3D_SAFE_CAP) bytes */
 cudaError_t launch_safe_distance(const uint8_t *tissue, int nx, int ny, int nz, uint8_t *radius,

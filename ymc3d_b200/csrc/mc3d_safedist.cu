@@ -271,6 +271,21 @@ __global__ void __launch_bounds__(256) one_tissue_kernel(int tissue, int nx, int
     }
 }
 
+/* Whether every voxel lies on a lateral face: all safe distances are 0 then, and rows
+ * padded to whole words would take up to four times the grid's own size. */
+bool all_on_faces(int nx, int ny) { return nx <= 2 || ny <= 2; }
+
+/* the cells of such a grid */
+__global__ void __launch_bounds__(256) on_faces_kernel(const uint8_t *__restrict__ t, int64_t plane,
+                                                       int nz, int nz_map,
+                                                       uint16_t *__restrict__ cells)
+{
+    const int64_t n = plane * nz_map;
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
+         v += (int64_t)gridDim.x * blockDim.x)
+        cells[v] = cell_of(t[min(v, plane * (nz - 1) + v % plane)], 0, 0);
+}
+
 /* blocks for `want` pieces of work: enough to fill the GPU several times */
 int grid_for(int64_t want) { return (int)(want < 148 * 32 ? (want > 0 ? want : 1) : 148 * 32); }
 
@@ -308,6 +323,7 @@ int64_t z_tiles(int nx, int ny, int nz)
 
 size_t safe_distance_scratch(int nx, int ny, int nz, bool index_map)
 {
+    if (all_on_faces(nx, ny)) return 0;
     const size_t map = (size_t)map_pitch(nx) * ny * ((size_t)nz + MC3D_SAFE_CAP);
     return map * (index_map ? 3 : 2);
 }
@@ -315,6 +331,8 @@ size_t safe_distance_scratch(int nx, int ny, int nz, bool index_map)
 cudaError_t launch_safe_distance(const uint8_t *tissue, int nx, int ny, int nz, uint8_t *radius,
                                  uint8_t *scratch, cudaStream_t stream)
 {
+    if (all_on_faces(nx, ny))
+        return cudaMemsetAsync(radius, 0, (size_t)nx * ny * ((size_t)nz + MC3D_SAFE_CAP), stream);
     const size_t map = safe_distance_scratch(nx, ny, nz, false) / 2;
     cudaError_t e = launch_d2(tissue, nx, ny, nz, nullptr, scratch, scratch + map, stream);
     if (e != cudaSuccess) return e;
@@ -335,6 +353,12 @@ cudaError_t launch_cells(const uint8_t *tissue, int nx, int ny, int nz, int one_
         const int64_t n = (int64_t)nx * ny * nz_map;
         one_tissue_kernel<<<grid_for((n + 255) / 256), 256, 0, stream>>>(one_tissue, nx, ny, nz_map,
                                                                          cells);
+        return cudaGetLastError();
+    }
+    if (all_on_faces(nx, ny)) {
+        const int64_t plane = (int64_t)nx * ny;
+        on_faces_kernel<<<grid_for((plane * nz_map + 255) / 256), 256, 0, stream>>>(
+            tissue, plane, nz, nz_map, cells);
         return cudaGetLastError();
     }
     const size_t map = safe_distance_scratch(nx, ny, nz, false) / 2;
