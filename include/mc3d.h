@@ -64,7 +64,14 @@ enum mc3d_math { MC3D_MATH_FAST = 0, MC3D_MATH_EXACT = 1, MC3D_MATH_F64 = 2 };
  * any refractive-index change or top or lateral face, so every reflection
  * happens in a one-voxel step; only the step counts in mc3d_totals differ.  The
  * mode applies to fast and FP64 math; exact math always steps at every face, and
- * so does a launch with a geometry of nx * ny * (nz + 63) >= 2^32 voxels. */
+ * so does a launch with a geometry of nx * ny * (nz + 63) >= 2^32 voxels.
+ *
+ * A job's photons are the same alone and beside other jobs, and with or without the
+ * absorption map, with two exceptions, both in merged steps.  Where other jobs use the
+ * same geometry with optical sets in which its tissues share their refractive indices
+ * differently, boxes end elsewhere and positions round differently.  And fast math
+ * rounds a scattering angle differently when it maps the absorption of a launch's only
+ * geometry.  The physics is the same in each. */
 enum mc3d_steps { MC3D_STEPS_MERGED = 0, MC3D_STEPS_VOXEL = 1 };
 
 /* Voxel geometry (geometry_t, src/mc3d_types.h:38-43), tissue indices as uint8

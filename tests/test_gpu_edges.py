@@ -12,7 +12,7 @@ import torch
 
 import ymc3d_b200 as m
 from conftest import ROOT
-from helpers import oracle_job, residual, safe_distance_bruteforce
+from helpers import oracle_job, residual, safe_distance_bruteforce, total_z
 from ymc3d_b200 import autotune, workloads
 
 pytestmark = pytest.mark.gpu
@@ -303,3 +303,30 @@ plan.execute()
 print(plan.read()[0].photons)
 """)
     assert int(out) == 1000
+
+
+# The absorption map changes no photon, nor does a second geometry in the launch: with one
+# exception.  The fast merged kernel that maps one geometry's absorption rounds the square
+# of the scattering cosine by itself, so a seeded run has tallies of its own there.
+@pytest.mark.parametrize("math,steps", MODES)
+def test_photons_with_and_without_the_map(table, math, steps):
+    g = m.Geometry(_blocks(11, (4, 5, 4), 3), 0.07, 0.07, 0.07)
+    other = m.Geometry(_blocks(12, (3, 3, 3), 3), 0.05, 0.06, 0.07)
+    p = m.OpticalProps.from_tissues([(0.3, 9.0, 0.9, 1.4), (0.5, 15.0, 0.7, 1.33),
+                                     (0.1, 6.0, 0.8, 1.4)])
+    job = m.Job(0, 0, 4000, 17, "uniform")
+    beside = m.Job(1, 0, 500, 18, "pencil")
+    kw = dict(table=table, math=math, steps=steps, photon_log=True)
+    off = m.run([g], [p], [job], **kw)[0]
+    on = m.run([g], [p], [job], absorption_map=True, **kw)[0]
+    _same(off, m.run([g, other], [p], [job, beside], **kw)[0])
+    batched = m.run([g, other], [p], [job, beside], absorption_map=True, **kw)[0]
+    _same(off, batched)
+    assert int(on.absorption.sum()) == on.totals["absorbed"] and residual(on.totals) == 0
+    if (math, steps) == ("fast", "merged"):
+        assert on.totals["steps"] != off.totals["steps"]
+        assert abs(total_z(on.totals, off.totals)) < 5
+        _same(on, m.run([g], [p], [job], absorption_map=True, block=64, **kw)[0])
+    else:
+        _same(on, off)
+        assert np.array_equal(on.absorption, batched.absorption)

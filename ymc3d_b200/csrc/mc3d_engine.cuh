@@ -8,8 +8,11 @@
  * photon slot of the reference does (src/mc3d_gpu.cu:74-111, 128-376) minus the
  * masked steps a frozen slot burns until the next host round trip.  Threads take
  * streams from a global counter, so the trajectories depend on (table, seed,
- * photons, streams) only -- never on the grid shape or on scheduling -- and the
- * tallies, being 64-bit integer sums, are bit-reproducible.
+ * photons, streams) and the math and step mode only -- never on the grid shape or on
+ * scheduling -- and the tallies, being 64-bit integer sums, are bit-reproducible.
+ * Fast merged steps know two things more of their launch: the optical sets that share
+ * a geometry, which decide where a box may end (cell_of), and whether it maps the
+ * absorption of a single geometry (scatter).
  *
  * Per-step physics follows src/mc3d_gpu.cu:175-340 operation for operation,
  * including its quirks (Fresnel denominator, 0/0 -> transmit at normal incidence,
@@ -45,7 +48,8 @@ namespace mc3d {
  * on its own; mad(a, b, c) is a b + c, one rounding with fast math and two with the
  * others.  The step uses these two wherever a product feeds a sum, so which
  * products fuse is written down and not the compiler's choice: the tallies do not
- * change with the code around an expression or with the register budget. */
+ * change with the code around an expression or with the register budget.  One kernel
+ * writes it down differently from the others (SPLIT_SIN2, see scatter). */
 
 /* Two values of one step side by side (its x and y axes): the fast policy computes on
  * both with one instruction, the others one after the other. */
