@@ -44,3 +44,12 @@ def has_gpu() -> bool:
         return torch.cuda.is_available()
     except Exception:
         return False
+
+
+def pytest_collection_modifyitems(items):
+    """The tests against the reference's own build (oracle/_ref, which needs its checkout)
+    fail where there is none.  They run last then, so that a run stopping at its first
+    failure has run every other test."""
+    if not (ROOT / "oracle" / "_ref").exists():
+        needs = {"run_reference", "ref_rng"}
+        items.sort(key=lambda item: not needs.isdisjoint(item.function.__code__.co_names))
