@@ -108,6 +108,7 @@ const int kMaxSharedTable = 192 * 1024;
 const int64_t kMaxAttempts = 4096;       /* seeding attempts per stream before giving up */
 const int64_t kMaxKeptSeeds = 1ll << 27; /* streams whose states a plan keeps (1 GiB) */
 const size_t kAlwaysKeptSeedBytes = 64u << 20;
+const size_t kTouchedArrayBytes = 1u << 20; /* outputs whose pages a read touches ahead */
 
 /* seeding-generator constants for multiplier `begin` (see mc3d_rng.h) */
 void make_seed_consts(uint32_t begin, mc3d_seed_consts *c)
@@ -193,16 +194,17 @@ void tissue_range(const uint8_t *tissue, int64_t nv, int *lo, int *hi)
 
 /* Write to every page of an output array without changing it.  Fresh pages of a caller's
  * array cost a fault each, 0.4 us, which would slow the copy into it to 2 GB/s; touched
- * while the GPU still works they cost nothing. */
+ * while the GPU still works they cost nothing.  An atomic write, so that none of the
+ * caller's own is lost. */
 void touch_pages(void *ptr, size_t bytes)
 {
     if (!ptr || !bytes) return;
-    volatile unsigned char *p = static_cast<volatile unsigned char *>(ptr);
+    unsigned char *p = static_cast<unsigned char *>(ptr);
     const int64_t pages = (int64_t)((bytes + 4095) / 4096);
     in_parallel(pages, 2048, [=](int64_t b, int64_t e) {
-        for (int64_t i = b; i < e; i++) p[i * 4096] = p[i * 4096];
+        for (int64_t i = b; i < e; i++) __atomic_fetch_or(p + i * 4096, 0, __ATOMIC_RELAXED);
     });
-    p[bytes - 1] = p[bytes - 1];
+    __atomic_fetch_or(p + bytes - 1, 0, __ATOMIC_RELAXED);
 }
 
 /* Rejected seeding attempts of one job from stream `first` on, in init_RNG's
@@ -871,14 +873,6 @@ int mc3d_plan_read(mc3d_plan *p, mc3d_out *out)
 {
     if (!p || !out) return fail(MC3D_ERR_ARG, "plan or out is NULL");
     CUDA_TRY(cudaSetDevice(p->device));
-    /* while the GPU works: the pages that will be written */
-    for (int j = 0; j < p->njobs; j++) {
-        const size_t nb = (size_t)p->job_bins[j] * sizeof(uint64_t);
-        touch_pages(out[j].drs, nb);
-        touch_pages(out[j].drs_sq, nb);
-        touch_pages(out[j].trans, nb);
-        if (p->d_amap) touch_pages(out[j].absorption, sizeof(uint64_t) * p->job_voxels[j]);
-    }
     /* Many small jobs: one copy of all tallies, up to 48 MB, handed out here instead of
      * three copies each (each waits for its end, about 20 us: 128 jobs of 64 x 64 bins
      * take 8.3 ms one by one, 6.0 ms at once). */
@@ -888,6 +882,20 @@ int mc3d_plan_read(mc3d_plan *p, mc3d_out *out)
         if (at_once) all.resize(3 * (size_t)p->total_bins);
     } catch (...) {
         at_once = false;
+    }
+    /* While the GPU works: the pages that will be written.  Not of small arrays that are
+     * copied one by one: a copy of theirs hides its faults behind its own latency, and where
+     * the GPU has finished already touching comes on top (600 jobs of 64 x 64 bins: 36.4 ms
+     * without, 39.5 with). */
+    for (int j = 0; j < p->njobs; j++) {
+        const size_t nb = (size_t)p->job_bins[j] * sizeof(uint64_t);
+        if (at_once || nb >= kTouchedArrayBytes) {
+            touch_pages(out[j].drs, nb);
+            touch_pages(out[j].drs_sq, nb);
+            touch_pages(out[j].trans, nb);
+        }
+        const size_t va = (size_t)p->job_voxels[j] * sizeof(uint64_t);
+        if (p->d_amap && va >= kTouchedArrayBytes) touch_pages(out[j].absorption, va);
     }
     CUDA_TRY(cudaDeviceSynchronize());
     std::vector<unsigned long long> tot((size_t)p->njobs * MC3D_NUM_TOTALS);
