@@ -44,9 +44,9 @@ OPS_JUMP = 8
 OPS_FRESNEL, SFU_FRESNEL = 37, 6
 FP32_LANES_PER_SM, SFU_LANES_PER_SM = 128, 16
 # DRAM bytes read + written by one photon-kernel launch of the layered workload (ncu
-# dram__bytes_read.sum + dram__bytes_write.sum = 114.0e6 + 4.1e6 on a 1e7-photon launch): the
+# dram__bytes_read.sum + dram__bytes_write.sum = 113.8e6 + 7.6e6 on a 1e7-photon launch): the
 # first touch of grid, packed cell map, table and tallies, and 8 bytes of stream state a photon
-TRAFFIC_BYTES_PER_LAUNCH, TRAFFIC_BYTES_PER_PHOTON = 38_100_000, 8
+TRAFFIC_BYTES_PER_LAUNCH, TRAFFIC_BYTES_PER_PHOTON = 41_400_000, 8
 
 
 def parse():

@@ -609,7 +609,7 @@ int mc3d_plan_create(mc3d_plan **plan_out, const mc3d_geom *geoms, int32_t ngeom
     /* ---- optical tables */
     /* three float4 per tissue; every derived value is the float the reference
      * computes per step (IEEE, no contraction: this file is built with
-     * -ffp-contract=off), except 1/mu_t, which only the fast kernel reads */
+     * -ffp-contract=off); 1/mu_t is correctly rounded, for exact math divides by it */
     std::vector<float4> tab(entries);
     for (int i = 0; i < nprops; i++)
         for (int t = 0; t < props[i].num_tissue_types; t++) {

@@ -29,7 +29,7 @@ struct GeomDev {
     int last_z;            /* last slice of the lookups: nz - 1, of the cells nz - 1 + MC3D_SAFE_CAP */
     float dx, dy, dz;      /* voxel size, float as in geometry_t (src/mc3d_types.h:38-43) */
     float Lx, Ly;          /* voxel size * count, computed in float */
-    float rdx, rdy, rdz;   /* 1 / voxel size (fast math only) */
+    float rdx, rdy, rdz;   /* 1 / voxel size, correctly rounded: exact math divides by them */
     int last_x, last_y;    /* nx - 1, ny - 1 */
     const uint8_t *tissue; /* nz*ny*nx, x fastest; 0 = air */
     const uint16_t *cells; /* tissue | box radius << 8, nz + MC3D_SAFE_CAP slices (merged) */

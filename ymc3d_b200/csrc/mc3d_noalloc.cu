@@ -279,7 +279,7 @@ extern "C" int mc3d_run_noalloc(const mc3d_geom *geom, const mc3d_props *props,
     P.seed = sc;
     int sms = 0, bps = 0;
     NA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const int block = 128; /* at most 28 KB of shared memory: no opt-in */
+    const int block = 128; /* at most 29 KB of shared memory: no opt-in */
     size_t smem = photon_smem(P.props_entries, 0, block);
     const auto kernel = photon_variant_wide(gd.nx, gd.ny, gd.nz) ? photon_kernel_noalloc_wide
                                                                  : photon_kernel_noalloc;
